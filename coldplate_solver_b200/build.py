@@ -4,7 +4,7 @@ the repository snapshot.
 The tile shape of the kernels is a compile-time constant, so each shape is
 its own library with the same C ABI: libcps.so (8 x 32 tiles, the default and
 the one the C++ drop-in links), libcps_t16.so (16 x 16) and libcps_t64.so
-(4 x 64).  The three compile in parallel.
+(4 x 64).  Their sources compile in parallel.
 
 ``--fmad=false``: the FP64 path keeps the reference's separate multiply and
 add roundings, so per-point values match the FP64 reference exactly; the
@@ -12,10 +12,12 @@ kernels are bound by memory and barrier latency, not by FP64 issue rate.
 """
 from __future__ import annotations
 
+import concurrent.futures
 import os
 import shutil
 import subprocess
 import sys
+import tempfile
 
 PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 REPO_DIR = os.path.dirname(PKG_DIR)
@@ -30,8 +32,9 @@ def lib_path(tile_j: int = 32) -> str:
     return LIB_PATH if tile_j == 32 else os.path.join(PKG_DIR, f"libcps_t{tile_j}.so")
 
 
-SOURCES = [os.path.join(PKG_DIR, "csrc", f) for f in ("cps_api.cu", "cps_noalloc.cu", "cps_thermal.cu", "cps_io.cpp",
-                                                              "cps_thermal_io.cpp")]
+SOURCES = [os.path.join(PKG_DIR, "csrc", f) for f in ("cps_api.cu", "cps_grid_f64.cu", "cps_grid_f32.cu",
+                                                            "cps_batch_f64.cu", "cps_batch_f32.cu", "cps_noalloc.cu",
+                                                            "cps_thermal.cu", "cps_io.cpp", "cps_thermal_io.cpp")]
 HEADERS = [os.path.join(PKG_DIR, "csrc", f) for f in os.listdir(os.path.join(PKG_DIR, "csrc")) if f.endswith(".cuh")]
 HEADERS.append(os.path.join(REPO_DIR, "include", "cps.h"))
 HEADERS.append(os.path.join(REPO_DIR, "include", "cps_thermal.h"))
@@ -64,16 +67,21 @@ def build(force: bool = False, verbose: bool = False) -> str:
     env = dict(os.environ)
     env.pop("CXX", None)
     env.pop("CC", None)
-    procs = []
-    for j in todo:
-        cmd = [nvcc(), *NVCC_FLAGS, f"-DCPS_TILE_J={j}", "-o", lib_path(j), *SOURCES]
-        if verbose:
-            cmd.insert(1, "-Xptxas=-v")
-            print(" ".join(cmd), file=sys.stderr)
-        procs.append((j, subprocess.Popen(cmd, env=env)))
-    failed = [j for j, p in procs if p.wait() != 0]
-    if failed:
-        raise RuntimeError(f"nvcc failed for tile widths {failed}")
+    flags = [f for f in NVCC_FLAGS if f != "-shared"] + (["-Xptxas=-v"] if verbose else [])
+    with tempfile.TemporaryDirectory() as tmp, concurrent.futures.ThreadPoolExecutor(os.cpu_count()) as pool:
+        def compile_one(j: int, src: str):
+            obj = os.path.join(tmp, f"{os.path.basename(src)}.{j}.o")
+            cmd = [nvcc(), *flags, f"-DCPS_TILE_J={j}", "-c", "-o", obj, src]
+            if verbose:
+                print(" ".join(cmd), file=sys.stderr)
+            return obj, subprocess.run(cmd, env=env).returncode
+
+        jobs = {j: [pool.submit(compile_one, j, src) for src in SOURCES] for j in todo}
+        for j, futures in jobs.items():
+            objs = [f.result() for f in futures]
+            if any(rc for _, rc in objs) or subprocess.run(
+                    [nvcc(), *NVCC_FLAGS, "-o", lib_path(j), *[o for o, _ in objs]], env=env).returncode:
+                raise RuntimeError(f"nvcc failed for tile width {j}")
     return LIB_PATH
 
 

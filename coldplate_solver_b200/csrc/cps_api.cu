@@ -33,7 +33,7 @@
 #include <vector>
 
 #include "../../include/cps.h"
-#include "cps_device.cuh"
+#include "cps_kernels.cuh"
 
 namespace {
 
@@ -83,208 +83,10 @@ struct cps_ctx {
   std::string err;
 };
 
-// Monitor: the outer loop's pressure-drop monitor and gate compiled in (a
-// separate instantiation: compiling it into the plain kernel slowed every
-// outer iteration by 60 % on B200).
-template <typename T, bool Monitor>
-__global__ void __launch_bounds__(cps::kThreads, CPS_MIN_BLOCKS) cps_grid_kernel(cps::DesignView d, cps::RunControl rc,
-                                                                cps::GridBarrier* bar, double* red) {
-  __shared__ double smem[(Monitor ? cps::kPlaneSums : cps::kRedWidth) * 8];
-  __shared__ cps::PseudoRun s_pr;
-  extern __shared__ __align__(128) char tile_smem[];
-  cps::GridGroup g{bar, red, rc.status, blockIdx.x, gridDim.x, 0u, 0ull};
-  if (!cps::tile_buffer_aligned(tile_smem, rc.status)) return;
-  cps::tma_barriers_init();
-  cps::load_pseudo(d, s_pr);
-  __syncthreads();
-  cps::SweepHint hint{2, 2, 2};
-  for (int it = 0; it < rc.n_outer; ++it) {
-    double out[8];
-    const int r = cps::outer_iteration<T, cps::GridGroup, Monitor>(
-        d, g, smem, tile_smem, out, it + 1 == rc.n_outer, rc.stop_on_conv != 0, rc.eps, rc.iter0 + it,
-        rc.dplog ? rc.dplog + (size_t)4 * it : nullptr, rc.dp_converged, &s_pr, &hint);
-    if (r < 0) return;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-      for (int k = 0; k < 8; ++k) rc.hist[(size_t)it * 8 + k] = out[k];
-      *rc.n_done = it + 1;
-    }
-    if (r == 1) return;
-  }
-}
-
-// Batched solves: each cluster takes the next design from the queue and runs
-// its outer iterations to convergence or to the item's budget.
-template <typename T, bool Pseudo>
-__global__ void __launch_bounds__(cps::kThreads) cps_cluster_kernel(const cps::BatchItem* __restrict__ items,
-                                                                   const int* __restrict__ order, int n_items,
-                                                                   int* queue, cps::BatchResult* results) {
-  __shared__ double smem[cps::kRedWidth * 8];
-  __shared__ double redbuf[2 * cps::kRedWidth];
-  __shared__ __align__(16) cps::BatchItem s_item;
-  __shared__ cps::PseudoRun s_pr;
-  __shared__ int s_next;
-  extern __shared__ __align__(128) char tile_smem[];
-  cps::cg::cluster_group cl = cps::cg::this_cluster();
-  cps::ClusterGroup g{redbuf, nullptr, cl.block_rank(), cl.num_blocks(), 0u};
-  if (!cps::tile_buffer_aligned(tile_smem, &results[0].status)) return;
-  cps::tma_barriers_init();
-  for (;;) {
-    if (g.rank == 0 && threadIdx.x == 0) s_next = atomicAdd(queue, 1);
-    cl.sync();
-    const int idx = *cl.map_shared_rank(&s_next, 0);
-    if (idx >= n_items) break;
-    const int id = order[idx];
-    {
-      const int* src = reinterpret_cast<const int*>(items + id);
-      int* dst = reinterpret_cast<int*>(&s_item);
-      for (int k = threadIdx.x; k < (int)(sizeof(cps::BatchItem) / sizeof(int)); k += blockDim.x) dst[k] = src[k];
-    }
-    __syncthreads();
-    const cps::BatchItem& item = s_item;
-    cps::load_pseudo(item.view, s_pr);
-    __syncthreads();
-    cps::BatchResult* res = results + id;
-    g.status = &res->status;
-    double out[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    int done = 0;
-    cps::SweepHint hint{2, 2, 2};
-    for (int it = 0; it < item.n_outer; ++it) {
-      const int r = cps::outer_iteration<T, cps::ClusterGroup, false, Pseudo>(
-          item.view, g, smem, tile_smem, out, it + 1 == item.n_outer, item.stop_on_conv != 0, item.eps, item.iter0 + it,
-          nullptr, nullptr, &s_pr, &hint);
-      done = it + 1;
-      if (g.rank == 0 && threadIdx.x == 0 && item.hist && it < item.hist_cap)
-        for (int k = 0; k < 8; ++k) item.hist[(size_t)it * 8 + k] = out[k];
-      if (r != 0) break;
-    }
-    if (g.rank == 0 && threadIdx.x == 0) {
-      res->n_done = done;
-      const double conv = cps::maxd(cps::maxd(out[0], out[1]), out[3]);
-      res->converged = (done > 0 && conv <= item.eps) ? 1 : 0;
-      for (int k = 0; k < 8; ++k) res->last[k] = out[k];
-    }
-    cl.sync();  // s_item, s_next and the reduction ring are reused next round
-  }
-  cl.sync();    // no CTA leaves while another may still read its shared memory
-}
-
-// Batched solves on groups of CTAs inside one cooperative launch: CTAs
-// [g*K, (g+1)*K) form group g, which takes designs from the queue one at a
-// time and runs each with the bounded software barrier of its own counter.
-// The group count sets how many designs are in flight (and so the in-flight
-// working set against the 126 MB L2); K sets how many CTAs share one design.
-template <typename T, bool Pseudo>
-__global__ void __launch_bounds__(cps::kThreads, CPS_MIN_BLOCKS) cps_group_kernel(const cps::BatchItem* __restrict__ items,
-                                                                    const int* __restrict__ order, int n_items,
-                                                                    int* queue, cps::BatchResult* results,
-                                                                    cps::GridBarrier* bars, double* rings,
-                                                                    int* slots, int group_ctas) {
-  __shared__ double smem[cps::kRedWidth * 8];
-  __shared__ __align__(16) cps::BatchItem s_item;
-  __shared__ cps::PseudoRun s_pr;
-  extern __shared__ __align__(128) char tile_smem[];
-  const unsigned grp = blockIdx.x / group_ctas;
-  int* slot = slots + 2 * grp;  // [0] next queue index, [1] group status before a design is assigned
-  cps::GridGroup g{bars + grp, rings + (size_t)grp * cps::kRedSlots * group_ctas * cps::kRedWidth, slot + 1,
-                   blockIdx.x % group_ctas, (unsigned)group_ctas, 0u, 0ull};
-  if (!cps::tile_buffer_aligned(tile_smem, &results[0].status)) return;
-  cps::tma_barriers_init();
-  for (;;) {
-    g.status = slot + 1;
-    if (g.rank == 0 && threadIdx.x == 0) slot[0] = atomicAdd(queue, 1);
-    if (!g.sync()) return;
-    const int idx = __ldcg(slot);
-    if (!g.sync()) return;  // every CTA has read the index before the leader takes the next one
-    if (idx >= n_items) return;
-    const int id = order[idx];
-    {
-      const int* src = reinterpret_cast<const int*>(items + id);
-      int* dst = reinterpret_cast<int*>(&s_item);
-      for (int k = threadIdx.x; k < (int)(sizeof(cps::BatchItem) / sizeof(int)); k += blockDim.x) dst[k] = src[k];
-    }
-    __syncthreads();
-    const cps::BatchItem& item = s_item;
-    cps::load_pseudo(item.view, s_pr);
-    __syncthreads();
-    cps::BatchResult* res = results + id;
-    g.status = &res->status;
-    double out[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    int done = 0;
-    cps::SweepHint hint{2, 2, 2};
-    for (int it = 0; it < item.n_outer; ++it) {
-      const int r = cps::outer_iteration<T, cps::GridGroup, false, Pseudo>(
-          item.view, g, smem, tile_smem, out, it + 1 == item.n_outer, item.stop_on_conv != 0, item.eps, item.iter0 + it,
-          nullptr, nullptr, &s_pr, &hint);
-      if (r < 0) return;  // a bounded wait expired; the design's status says so
-      done = it + 1;
-      if (g.rank == 0 && threadIdx.x == 0 && item.hist && it < item.hist_cap)
-        for (int k = 0; k < 8; ++k) item.hist[(size_t)it * 8 + k] = out[k];
-      if (r != 0) break;
-    }
-    if (g.rank == 0 && threadIdx.x == 0) {
-      res->n_done = done;
-      const double conv = cps::maxd(cps::maxd(out[0], out[1]), out[3]);
-      res->converged = (done > 0 && conv <= item.eps) ? 1 : 0;
-      for (int k = 0; k < 8; ++k) res->last[k] = out[k];
-    }
-    __syncthreads();  // s_item is reloaded next round
-  }
-}
-
-// Batched solves in waves: one design per group, groups sized to their
-// designs.  CTAs [first[g], first[g+1]) form group g and run design which[g]
-// to convergence or to its budget with the bounded software barrier of their
-// own counter; their reduction ring starts at first[g] ring rows.
-template <typename T, bool Pseudo>
-__global__ void __launch_bounds__(cps::kThreads, CPS_MIN_BLOCKS) cps_wave_kernel(const cps::BatchItem* __restrict__ items,
-                                                                   const int* __restrict__ first,
-                                                                   const int* __restrict__ which, int groups,
-                                                                   cps::BatchResult* results,
-                                                                   cps::GridBarrier* bars, double* rings) {
-  __shared__ double smem[cps::kRedWidth * 8];
-  __shared__ __align__(16) cps::BatchItem s_item;
-  __shared__ cps::PseudoRun s_pr;
-  extern __shared__ __align__(128) char tile_smem[];
-  if (!cps::tile_buffer_aligned(tile_smem, &results[which[0]].status)) return;
-  cps::tma_barriers_init();
-  int lo = 0, hi = groups;  // first[lo] <= blockIdx.x < first[lo + 1]
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (first[mid] <= (int)blockIdx.x) lo = mid; else hi = mid;
-  }
-  const int grp = lo, K = first[grp + 1] - first[grp], id = which[grp];
-  {
-    const int* src = reinterpret_cast<const int*>(items + id);
-    int* dst = reinterpret_cast<int*>(&s_item);
-    for (int k = threadIdx.x; k < (int)(sizeof(cps::BatchItem) / sizeof(int)); k += blockDim.x) dst[k] = src[k];
-  }
-  __syncthreads();
-  const cps::BatchItem& item = s_item;
-  cps::load_pseudo(item.view, s_pr);
-  __syncthreads();
-  cps::BatchResult* res = results + id;
-  cps::GridGroup g{bars + grp, rings + (size_t)first[grp] * cps::kRedSlots * cps::kRedWidth, &res->status,
-                   blockIdx.x - (unsigned)first[grp], (unsigned)K, 0u, 0ull};
-  double out[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  int done = 0;
-  cps::SweepHint hint{2, 2, 2};
-  for (int it = 0; it < item.n_outer; ++it) {
-    const int r = cps::outer_iteration<T, cps::GridGroup, false, Pseudo>(
-        item.view, g, smem, tile_smem, out, it + 1 == item.n_outer, item.stop_on_conv != 0, item.eps, item.iter0 + it,
-        nullptr, nullptr, &s_pr, &hint);
-    if (r < 0) return;  // a bounded wait expired; the design's status says so
-    done = it + 1;
-    if (g.rank == 0 && threadIdx.x == 0 && item.hist && it < item.hist_cap)
-      for (int k = 0; k < 8; ++k) item.hist[(size_t)it * 8 + k] = out[k];
-    if (r != 0) break;
-  }
-  if (g.rank == 0 && threadIdx.x == 0) {
-    res->n_done = done;
-    const double conv = cps::maxd(cps::maxd(out[0], out[1]), out[3]);
-    res->converged = (done > 0 && conv <= item.eps) ? 1 : 0;
-    for (int k = 0; k < 8; ++k) res->last[k] = out[k];
-  }
-}
+CPS_GRID_KERNELS(extern, double)
+CPS_GRID_KERNELS(extern, float)
+CPS_BATCH_KERNELS(extern, double)
+CPS_BATCH_KERNELS(extern, float)
 
 // samplePlaneAtX (postprocessing.cpp:62-230) for one plane, one CTA: every row's
 // contribution is evaluated with the reference's expressions; the five sums are
@@ -497,10 +299,11 @@ void set_step_inputs(cps_ctx* c, double Uin) {
   c->view.maxVel = 3.0 * std::max(std::fabs(Uin), 0.1);  // iterations.cpp:104
 }
 
-const void* grid_kernel_for(int precision, bool monitor = false) {
-  if (monitor)
-    return precision == CPS_MIXED ? (const void*)cps_grid_kernel<float, true> : (const void*)cps_grid_kernel<double, true>;
-  return precision == CPS_MIXED ? (const void*)cps_grid_kernel<float, false> : (const void*)cps_grid_kernel<double, false>;
+const void* grid_kernel_for(int precision, bool monitor = false, bool pseudo = false) {
+  const bool mixed = precision == CPS_MIXED;
+  if (monitor) return mixed ? (const void*)cps_grid_kernel<float, true, true> : (const void*)cps_grid_kernel<double, true, true>;
+  if (pseudo) return mixed ? (const void*)cps_grid_kernel<float, false, true> : (const void*)cps_grid_kernel<double, false, true>;
+  return mixed ? (const void*)cps_grid_kernel<float, false, false> : (const void*)cps_grid_kernel<double, false, false>;
 }
 
 // Dynamic shared memory of the persistent kernels (tile staging buffers).
@@ -542,7 +345,7 @@ cps_status run(cps_ctx* c, int n_outer, int stop_on_conv, double eps, cps_step_o
       return CPS_ERR_CUDA;
     void* args[] = {&c->view, &rc, &c->bar, &c->red};
     if (!cuda_ok(c, cudaEventRecord(c->ev0, c->stream), "event")) return CPS_ERR_CUDA;
-    if (!cuda_ok(c, cudaLaunchCooperativeKernel(grid_kernel_for(c->precision, monitor), dim3(c->grid), dim3(cps::kThreads),
+    if (!cuda_ok(c, cudaLaunchCooperativeKernel(grid_kernel_for(c->precision, monitor, c->view.pseudo != 0), dim3(c->grid), dim3(cps::kThreads),
                                                 args, tile_smem_for(c->precision), c->stream), "cooperative launch"))
       return CPS_ERR_CUDA;
     if (!cuda_ok(c, cudaEventRecord(c->ev1, c->stream), "event")) return CPS_ERR_CUDA;
@@ -774,6 +577,8 @@ cps_status cps_create(const cps_desc* d, cps_ctx** out) {
   v.Fcy = convScale * d->rho * d->hx;
   v.relax = (1.0 - d->uvAlpha) / d->uvAlpha;
   const double tolsq = d->momentumTol * d->momentumTol;
+  v.rUvAlpha = 1.0 / d->uvAlpha;
+  v.pStop = cps::pcg_stop(d->pTol);
   v.thrU = tolsq * (double)((d->M - 1) * (d->N - 2));
   v.thrV = tolsq * (double)((d->M - 2) * (d->N - 1));
   v.u = field_ptr(c, kU); v.v = field_ptr(c, kV); v.p = field_ptr(c, kP); v.pc = field_ptr(c, kPc);
@@ -802,6 +607,7 @@ cps_status cps_create(const cps_desc* d, cps_ctx** out) {
   int per_sm = 0, sms = 0;
   if (!allow_smem(c, grid_kernel_for(d->precision), tile_smem_for(d->precision)) ||
       !allow_smem(c, grid_kernel_for(d->precision, true), tile_smem_for(d->precision)) ||
+      !allow_smem(c, grid_kernel_for(d->precision, false, true), tile_smem_for(d->precision)) ||
       !cuda_ok(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, grid_kernel_for(d->precision),
                                                                 cps::kThreads, tile_smem_for(d->precision)),
                "occupancy") ||

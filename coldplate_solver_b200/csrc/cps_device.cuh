@@ -61,6 +61,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <cooperative_groups.h>
+#include <math.h>
 #include <stdint.h>
 
 namespace cps {
@@ -141,6 +142,8 @@ struct DesignView {
   double hx, hy, rho, uvAlpha, pAlpha, pTol;
   double vol, De, Dn, sinkDiag, Fcx, Fcy, relax;  // Fcx = cs*rho*hy, Fcy = cs*rho*hx, relax = (1-uvA)/uvA
   double thrU, thrV;                              // momTol^2 * nU, momTol^2 * nV
+  double rUvAlpha;                                // 1 / uvAlpha, rounded to nearest
+  double pStop;                                   // pcg_stop(pTol): sqrt(x) < pTol exactly when x < pStop
   double Uin, maxVel;
   double *u, *v, *p, *pc, *us, *vs, *dE, *dN, *alpha, *gamma;
   long long planeStride;                          // elements between coefficient planes
@@ -229,6 +232,16 @@ struct BatchResult {
   double last[8];     // diagnostics of the last iteration
 };
 
+// The smallest x >= 0 whose rounded square root is at least pTol: the PCG's
+// test sqrt(|r|^2) < pTol without a square root per iteration and thread.
+inline double pcg_stop(double pTol) {
+  if (!(pTol > 0.0)) return 0.0;
+  double x = pTol * pTol;
+  while (x > 0.0 && sqrt(x) >= pTol) x = nextafter(x, 0.0);
+  while (sqrt(x) < pTol && x < HUGE_VAL) x = nextafter(x, HUGE_VAL);
+  return x;
+}
+
 // Monotonic arrival counter of the grid barrier; zeroed before every launch.
 struct GridBarrier {
   unsigned long long count;
@@ -240,6 +253,40 @@ struct GridBarrier {
 __device__ __forceinline__ double maxd(double a, double b) { return (a < b) ? b : a; }
 __device__ __forceinline__ double mind(double a, double b) { return (b < a) ? b : a; }
 __device__ __forceinline__ double clampd(double v, double lo, double hi) { return (v < lo) ? lo : (hi < v) ? hi : v; }
+
+// ---------------------------------------------------------------------------
+// Correctly rounded division without a branch.  The quotient is corrected once
+// from its exact remainder (Markstein, IBM J. Res. Dev. 34, 1990): with y =
+// 1/b rounded to nearest, q = a y and r = a - b q (exact under fma), q + r y
+// is a/b rounded to nearest, the value `/` returns.  y comes from two Newton
+// steps on the hardware's reciprocal approximation and is shared by divisions
+// with a divisor in common.
+//
+// Why: `/` guards its operands with a branch, so consecutive divisions of a
+// thread do not overlap, and a zero numerator (solid cells, fields not yet
+// reached from the zero state) takes its out-of-line path.  Measured on B200,
+// divisions per SM and clock at 512 threads: `/` 3.5, `/` with zero numerators
+// 0.9, this 6.0 either way; per division of one warp 130, 434 and 35 clocks.
+//
+// Range: y must be normal (2^-1000 <= |b| <= 2^1000 here: the divisors are
+// relaxed momentum diagonals >= 1e-10 and pressure diagonals >= 1e-20).  For
+// quotients below 2^-960 the remainder may underflow and the last bit is not
+// guaranteed; an infinite numerator or an overflowing quotient gives q.
+// ---------------------------------------------------------------------------
+// One Newton step of y towards 1/b.
+__device__ __forceinline__ double recip_step(double b, double y) { return __fma_rn(y, __fma_rn(-b, y, 1.0), y); }
+__device__ __forceinline__ double recip(double b) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+  return recip_step(b, recip_step(b, y));
+}
+// a / b with y = recip(b).
+__device__ __forceinline__ double div_rn(double a, double b, double y) {
+  const double q = a * y;
+  const double v = __fma_rn(__fma_rn(-b, q, a), y, q);
+  return (__double2hiint(v) & 0x7ff00000) == 0x7ff00000 ? q : v;
+}
+__device__ __forceinline__ double div_rn(double a, double b) { return div_rn(a, b, recip(b)); }
 
 // ---------------------------------------------------------------------------
 // Pseudo-transient term and CFL controllers
@@ -968,6 +1015,7 @@ __device__ __forceinline__ double sou_correction(const DesignView& d, const X& x
 // get the same bits.
 struct MomRow {
   double cE, cW, cN, cS, aP, Sp, velCur;
+  double rAP;  // recip(aP), from the reciprocal of aP0 that dOut needs
   bool hasE, hasW, hasN, hasS;
 };
 
@@ -1003,12 +1051,14 @@ __device__ __forceinline__ MomRow momentum_row(const DesignView& d, const Layout
   const double brinkmanDrag = alphaLocal * d.vol;
   double aP0 = sumA + (Fe - Fw + Fn - Fs) + transCoeff + d.sinkDiag + brinkmanDrag;
   aP0 = maxd(aP0, 1e-10);
-  m.aP = aP0 / d.uvAlpha;
+  m.aP = div_rn(aP0, d.uvAlpha, d.rUvAlpha);
   double Sp = IsU ? (L.p(i, j) - L.p(i, j + 1)) * d.hy : (L.p(i, j) - L.p(i + 1, j)) * d.hx;
   Sp += transCoeff * m.velCur;
   Sp += d.relax * aP0 * m.velCur;
   if (d.conv == 1) Sp += sou_correction<IsU>(d, X, i, j, Fe, Fw, Fn, Fs);
-  dOut = (IsU ? d.hy : d.hx) / aP0;
+  const double rAP0 = recip(aP0);
+  dOut = div_rn(IsU ? d.hy : d.hx, aP0, rAP0);
+  m.rAP = recip_step(m.aP, d.uvAlpha * rAP0);
   const int iHi = IsU ? M - 1 : M - 2, jHi = IsU ? N - 2 : N - 1;
   m.hasE = j + 1 <= jHi;
   m.hasW = j - 1 >= 1;
@@ -1076,10 +1126,10 @@ __device__ __forceinline__ double assemble_point(const DesignView& d, const Layo
   if (storeRow)
     store_row<IsU, T>(d, o, (T)m.cE, (T)m.cW, (T)m.cN, (T)m.cS, (T)m.aP, kMixed ? (T)r : (T)m.Sp);
   if (kMixed) {
-    (IsU ? w.xU1 : w.xV1)[o] = (T)(r / m.aP);
+    (IsU ? w.xU1 : w.xV1)[o] = (T)div_rn(r, m.aP, m.rAP);
     return r * r;
   }
-  (IsU ? w.xU1 : w.xV1)[o] = (T)(m.velCur + r / m.aP);
+  (IsU ? w.xU1 : w.xV1)[o] = (T)(m.velCur + div_rn(r, m.aP, m.rAP));
   return r * r;
 }
 
@@ -1108,7 +1158,7 @@ __device__ __forceinline__ double sweep2_point(const DesignView& d, const Layout
   if (m.hasE) Ax += (double)cE * (double)xin[o + 1];
   if (m.hasN) Ax += (double)cN * (double)xin[o + P];
   const double r = (double)bt - Ax;
-  xout[o] = (T)(x0 + r / aP);
+  xout[o] = (T)(x0 + div_rn(r, aP));
   return r * r;
 }
 
@@ -1220,7 +1270,7 @@ __device__ __forceinline__ double sweep_point_staged(const DesignView& d, const 
   if (j + 1 <= jHi) Ax += (double)c[0](i, j) * (double)X(i, j + 1);
   if (i + 1 <= iHi) Ax += (double)c[2](i, j) * (double)X(i + 1, j);
   const double r = (double)(IsU ? L.bu : L.bv)(i, j) - Ax;
-  xout[(size_t)i * P + j] = (T)(x0 + r / aP);
+  xout[(size_t)i * P + j] = (T)(x0 + div_rn(r, aP));
   return r * r;
 }
 
@@ -1242,7 +1292,7 @@ __device__ __forceinline__ double sweep_point(const DesignView& d, int i, int j,
   if (j + 1 <= jHi) Ax += (double)c[o] * (double)xin[o + 1];
   if (i + 1 <= iHi) Ax += (double)c[o + 2 * ps] * (double)xin[o + P];
   const double r = (double)(IsU ? w.bU : w.bV)[o] - Ax;
-  xout[o] = (T)(x0 + r / aP);
+  xout[o] = (T)(x0 + div_rn(r, aP));
   return r * r;
 }
 
@@ -1301,12 +1351,12 @@ __device__ int pcg_two_reductions(const DesignView& d, Group& g, double* smem, d
       const double r = (double)rt;
       s2[0] += r * r;
       const double dg = (double)dgo;
-      const T z = (T)((fabs(dg) > 1e-20) ? r / dg : r);
+      const T z = (T)((fabs(dg) > 1e-20) ? div_rn(r, dg) : r);
       w.pz[o] = z;
       s2[1] += r * (double)z;
     });
     if (!g.template sync_reduce<2, 0u>(s2, smem)) return -1;
-    if (sqrt(s2[0]) < d.pTol) break;
+    if (s2[0] < d.pStop) break;
     const double rzPrev = rz;
     rz = s2[1];
     beta = rz / rzPrev;
@@ -1413,13 +1463,13 @@ __device__ int pcg_resident(const DesignView& d, Group& g, double* smem, double 
       const double rr = (double)rt;
       s2[0] += rr * rr;
       const double dgd = (double)dg[u];
-      const T zz = (T)((fabs(dgd) > 1e-20) ? rr / dgd : rr);
+      const T zz = (T)((fabs(dgd) > 1e-20) ? div_rn(rr, dgd) : rr);
       z[u] = zz;
       w.pz[oo[u]] = zz;
       s2[1] += rr * (double)zz;
     }
     if (!g.template sync_reduce<2, 0u>(s2, smem)) return -1;
-    if (sqrt(s2[0]) < d.pTol) break;
+    if (s2[0] < d.pStop) break;
     const double rzPrev = rz;
     rz = s2[1];
     beta = rz / rzPrev;
@@ -1614,13 +1664,13 @@ __device__ int pcg_smem(const DesignView& d, Group& g, double* smem, char* tbuf,
       const double r = (double)rt;
       s2[0] += r * r;
       const double dgd = diag(k, i, j);
-      const T zt = (T)((fabs(dgd) > 1e-20) ? r / dgd : r);
+      const T zt = (T)((fabs(dgd) > 1e-20) ? div_rn(r, dgd) : r);
       S.z[k][th] = zt;
       w.pz[o] = zt;
       s2[1] += r * (double)zt;
     }
     if (!g.template sync_reduce<2, 0u>(s2, smem)) return -1;
-    if (sqrt(s2[0]) < d.pTol) break;
+    if (s2[0] < d.pStop) break;
     const double rzPrev = rz;
     rz = s2[1];
     beta = rz / rzPrev;
@@ -1662,7 +1712,7 @@ __device__ int pcg_single_reduction(const DesignView& d, Group& g, double* smem,
   if (d.maxPIter <= 0) return 0;
   auto inv_diag = [&](size_t q, double r) -> double {
     const double dg = (double)w.pdiag[q];
-    return (fabs(dg) > 1e-20) ? r / dg : r;
+    return (fabs(dg) > 1e-20) ? div_rn(r, dg) : r;
   };
   // w0 = A u0 and delta0 = (w0, u0) come from phase C
   double gam = gamma0;
@@ -1715,7 +1765,7 @@ __device__ int pcg_single_reduction(const DesignView& d, Group& g, double* smem,
       red[2] += (double)wt * uc;
     });
     if (!g.template sync_reduce<3, 0u>(red, smem)) return -1;
-    if (sqrt(red[0]) < d.pTol) break;
+    if (red[0] < d.pStop) break;
     if (k + 1 >= d.maxPIter) { k = d.maxPIter; break; }
     const double gNew = red[1];
     const double bNew = gNew / gam;
@@ -1958,7 +2008,7 @@ __device__ bool mass_phase(const DesignView& d, Group& g, double* smem, char* tb
             double aP = aE + aW + aN + aS;
             if (aP < 1e-20) aP = 1.0;
             const double rr = (double)(T)b, dd = (double)(T)aP;
-            z = (double)(T)((fabs(dd) > 1e-20) ? rr / dd : rr);
+            z = (double)(T)((fabs(dd) > 1e-20) ? div_rn(rr, dd) : rr);
           }
           z0.ref(k) = z;
         }
@@ -2004,8 +2054,8 @@ __device__ bool mass_phase(const DesignView& d, Group& g, double* smem, char* tb
           const T rt = (T)b;
           w.pr[o] = rt;
           w.px[o] = (T)0.0;
-          const double rr = (double)rt, dd = (double)dg;
-          const T z = (T)((fabs(dd) > 1e-20) ? rr / dd : rr);
+          const double rr = (double)rt;
+          const T z = (T)z0(i, j);  // formed from the same stored values above
           if (d.pcgSingleReduction) {
             w.cU[o + d.planeStride] = z;  // u0 = M^-1 r0 of the single-reduction recurrences
           } else {
@@ -2234,8 +2284,9 @@ __device__ __forceinline__ bool tile_buffer_aligned(const char* dyn, int* status
 }
 
 // ---------------------------------------------------------------------------
-// One outer iteration for one design on group g; out[8] receives the step
-// diagnostics.  tbuf: tile_smem_bytes<T>() of shared memory.  iter is the
+// One outer iteration for one design on group g; out[8], in shared memory (held
+// in registers it cost every thread 16 of them through the PCG), receives the
+// step diagnostics from thread 0, the only thread that may read them back.  tbuf: tile_smem_bytes<T>() of shared memory.  iter is the
 // outer loop's iteration index of this step.  With Monitor (compiled in for
 // the single-design kernel only) and d.dpMonitor, dplog (may be null) receives
 // its four pressure drops and *dpConverged is set when the pressure-drop gate
@@ -2247,7 +2298,7 @@ __device__ __forceinline__ bool tile_buffer_aligned(const char* dyn, int* status
 // because a device-side wait failed.
 // ---------------------------------------------------------------------------
 template <typename T, class Group, bool Monitor = false, bool Pseudo = true>
-__device__ int outer_iteration(const DesignView& d, Group& g, double* smem, char* tbuf, double (&out)[8],
+__device__ int outer_iteration(const DesignView& d, Group& g, double* smem, char* tbuf, double* out,
                                bool lastIter, bool stopOnConv, double eps, int iter = 0, double* dplog = nullptr,
                                int* dpConverged = nullptr, PseudoRun* pr = nullptr, SweepHint* hint = nullptr) {
   const Inner<T>& w = inner<T>(d);
@@ -2373,29 +2424,31 @@ __device__ int outer_iteration(const DesignView& d, Group& g, double* smem, char
   double rc[7] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
   if (!mass_phase<T>(d, g, smem, tbuf, xfU, xfV, (kU & 1) ? kTmXU1_C : kTmXU0_C, (kV & 1) ? kTmXV1_C : kTmXV0_C, rc))
     return -1;
-  out[0] = rc[0];
-  out[1] = rc[1];
-  out[2] = rc[2];
-  out[3] = rc[3];
-  out[6] = kU;
-  out[7] = kV;
   // std::max({residU, residV, residMass}) (iterations.cpp:525); the stop test
   // uses the mass imbalance over the pressure unknowns.
-  double e = out[0];
-  if (e < out[1]) e = out[1];
-  if (e < out[2]) e = out[2];
-  out[4] = e;
-  const double conv = maxd(maxd(out[0], out[1]), out[3]);
+  double e = rc[0];
+  if (e < rc[1]) e = rc[1];
+  if (e < rc[2]) e = rc[2];
+  const double conv = maxd(maxd(rc[0], rc[1]), rc[3]);
   // The max reductions drop NaN the way std::max does, so non-finite values
   // are flagged explicitly.
-  const bool finite = isfinite(e) && isfinite(out[3]) && rc[4] == 0.0;
+  const bool finite = isfinite(e) && isfinite(rc[3]) && rc[4] == 0.0;
   if (!finite && g.rank == 0 && threadIdx.x == 0 && g.status) atomicCAS(g.status, kStatusOk, kStatusDiverged);
   const bool stop = lastIter || !finite || (stopOnConv && conv <= eps);
+  if (threadIdx.x == 0) {
+    out[0] = rc[0];
+    out[1] = rc[1];
+    out[2] = rc[2];
+    out[3] = rc[3];
+    out[4] = e;
+    out[6] = kU;
+    out[7] = kV;
+  }
   // The CFL controllers (SIMPLE.cpp:321-327).  Every CTA's thread 0 updates its
   // copy from the same reduced residuals; the barriers before the next phase A
   // publish it to the CTA.
   if (Pseudo && d.pseudo && pr && threadIdx.x == 0) {
-    pseudo_update(d, *pr, d.serUseMax ? out[4] : out[2], iter);
+    pseudo_update(d, *pr, d.serUseMax ? e : rc[2], iter);
     if (g.rank == 0 && d.pseudoState) {
       d.pseudoState[0] = pr->cfl;
       d.pseudoState[1] = pr->prev;
@@ -2407,7 +2460,7 @@ __device__ int outer_iteration(const DesignView& d, Group& g, double* smem, char
   if (d.pcgSingleReduction) {
     const int its = pcg_single_reduction<T>(d, g, smem, rc[5], rc[6]);
     if (its < 0) return -1;
-    out[5] = its;
+    if (threadIdx.x == 0) out[5] = its;
   } else {
     const int tiles = ((M - 1 + kTileI - 1) / kTileI) * ((N - 1 + kTileJ - 1) / kTileJ);
     constexpr int kS = SmemTiles<T>::value;
@@ -2421,7 +2474,7 @@ __device__ int outer_iteration(const DesignView& d, Group& g, double* smem, char
     else
       its = pcg_two_reductions<T>(d, g, smem, rc[5], rc[6]);
     if (its < 0) return -1;
-    out[5] = its;
+    if (threadIdx.x == 0) out[5] = its;
     if (hint) hint->kP = its;
   }
   // ---- D: pressure and velocity correction ----

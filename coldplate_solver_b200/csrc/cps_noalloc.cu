@@ -65,11 +65,11 @@ cps_status fail(cps_status s, const std::string& m) {
 __global__ void __launch_bounds__(cps::kThreads, CPS_MIN_BLOCKS) cps_noalloc_kernel(cps::DesignView d, cps::RunControl rc,
                                                                       cps::GridBarrier* bar, double* red) {
   __shared__ double smem[cps::kRedWidth * 8];
+  __shared__ double out[8];
   extern __shared__ __align__(128) char tile_smem[];
   cps::GridGroup g{bar, red, rc.status, blockIdx.x, gridDim.x, 0u, 0ull};  // no tensor maps: element-wise staging
   cps::SweepHint hint{2, 2, 2};
   for (int it = 0; it < rc.n_outer; ++it) {
-    double out[8];
     const int r = cps::outer_iteration<double>(d, g, smem, tile_smem, out, it + 1 == rc.n_outer,
                                                rc.stop_on_conv != 0, rc.eps, 0, nullptr, nullptr, nullptr, &hint);
     if (r < 0) return;
@@ -144,6 +144,8 @@ extern "C" cps_status cps_solve_noalloc(const cps_desc* desc, int pitch, const d
   w.Fcy = convScale * d.rho * d.hx;
   w.relax = (1.0 - d.uvAlpha) / d.uvAlpha;
   const double tolsq = d.momentumTol * d.momentumTol;
+  w.rUvAlpha = 1.0 / d.uvAlpha;
+  w.pStop = cps::pcg_stop(d.pTol);
   w.thrU = tolsq * (double)((d.M - 1) * (d.N - 2));
   w.thrV = tolsq * (double)((d.M - 2) * (d.N - 1));
   w.Uin = inletVelocity;
