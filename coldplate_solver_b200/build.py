@@ -32,9 +32,10 @@ def lib_path(tile_j: int = 32) -> str:
     return LIB_PATH if tile_j == 32 else os.path.join(PKG_DIR, f"libcps_t{tile_j}.so")
 
 
-SOURCES = [os.path.join(PKG_DIR, "csrc", f) for f in ("cps_api.cu", "cps_grid_f64.cu", "cps_grid_f32.cu",
-                                                            "cps_batch_f64.cu", "cps_batch_f32.cu", "cps_noalloc.cu",
-                                                            "cps_thermal.cu", "cps_io.cpp", "cps_thermal_io.cpp")]
+SOURCES = [os.path.join(PKG_DIR, "csrc", f) for f in (
+    "cps_grid_f64.cu", "cps_grid_f32.cu", "cps_grid_opt_f64.cu", "cps_grid_opt_f32.cu", "cps_batch_f64.cu",
+    "cps_batch_f32.cu", "cps_batch_opt_f64.cu", "cps_batch_opt_f32.cu", "cps_api.cu", "cps_noalloc.cu",
+    "cps_thermal.cu", "cps_io.cpp", "cps_thermal_io.cpp")]
 HEADERS = [os.path.join(PKG_DIR, "csrc", f) for f in os.listdir(os.path.join(PKG_DIR, "csrc")) if f.endswith(".cuh")]
 HEADERS.append(os.path.join(REPO_DIR, "include", "cps.h"))
 HEADERS.append(os.path.join(REPO_DIR, "include", "cps_thermal.h"))

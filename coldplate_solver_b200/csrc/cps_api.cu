@@ -85,8 +85,12 @@ struct cps_ctx {
 
 CPS_GRID_KERNELS(extern, double)
 CPS_GRID_KERNELS(extern, float)
+CPS_GRID_OPTION_KERNELS(extern, double)
+CPS_GRID_OPTION_KERNELS(extern, float)
 CPS_BATCH_KERNELS(extern, double)
 CPS_BATCH_KERNELS(extern, float)
+CPS_BATCH_OPTION_KERNELS(extern, double)
+CPS_BATCH_OPTION_KERNELS(extern, float)
 
 // samplePlaneAtX (postprocessing.cpp:62-230) for one plane, one CTA: every row's
 // contribution is evaluated with the reference's expressions; the five sums are
@@ -299,11 +303,34 @@ void set_step_inputs(cps_ctx* c, double Uin) {
   c->view.maxVel = 3.0 * std::max(std::fabs(Uin), 0.1);  // iterations.cpp:104
 }
 
-const void* grid_kernel_for(int precision, bool monitor = false, bool pseudo = false) {
-  const bool mixed = precision == CPS_MIXED;
-  if (monitor) return mixed ? (const void*)cps_grid_kernel<float, true, true> : (const void*)cps_grid_kernel<double, true, true>;
-  if (pseudo) return mixed ? (const void*)cps_grid_kernel<float, false, true> : (const void*)cps_grid_kernel<double, false, true>;
-  return mixed ? (const void*)cps_grid_kernel<float, false, false> : (const void*)cps_grid_kernel<double, false, false>;
+// The single-design kernels of a storage type: one per PCG form on the default
+// path, then the ones that carry every option, without and with the monitor.
+template <typename T>
+const void* grid_kernel(int k) {
+  switch (k) {
+    case 0: return (const void*)cps_grid_kernel<T, false, false, cps::kFew>;
+    case 1: return (const void*)cps_grid_kernel<T, false, false, cps::kMany>;
+    case 2: return (const void*)cps_grid_kernel<T, false, false, cps::kLarge>;
+    case 3: return (const void*)cps_grid_kernel<T, false, true, cps::kAll>;
+    default: return (const void*)cps_grid_kernel<T, true, true, cps::kAll>;
+  }
+}
+constexpr int kGridKernels = 5;
+const void* grid_kernel_of(int precision, int k) {
+  return precision == CPS_MIXED ? grid_kernel<float>(k) : grid_kernel<double>(k);
+}
+
+// Whether a design needs a kernel that carries the options.
+bool has_options(const cps::DesignView& v) {
+  return v.pseudo != 0 || v.momExplicit != 0 || v.pcgSingleReduction != 0 || v.stageSweeps != 0;
+}
+
+const void* grid_kernel_for(const cps_ctx* c) {
+  if (c->view.dpMonitor) return grid_kernel_of(c->precision, 4);
+  if (has_options(c->view)) return grid_kernel_of(c->precision, 3);
+  const int form = c->precision == CPS_MIXED ? cps::pcg_form<float>(c->M, c->N, c->grid)
+                                             : cps::pcg_form<double>(c->M, c->N, c->grid);
+  return grid_kernel_of(c->precision, form == cps::kFew ? 0 : form == cps::kMany ? 1 : 2);
 }
 
 // Dynamic shared memory of the persistent kernels (tile staging buffers).
@@ -345,7 +372,7 @@ cps_status run(cps_ctx* c, int n_outer, int stop_on_conv, double eps, cps_step_o
       return CPS_ERR_CUDA;
     void* args[] = {&c->view, &rc, &c->bar, &c->red};
     if (!cuda_ok(c, cudaEventRecord(c->ev0, c->stream), "event")) return CPS_ERR_CUDA;
-    if (!cuda_ok(c, cudaLaunchCooperativeKernel(grid_kernel_for(c->precision, monitor, c->view.pseudo != 0), dim3(c->grid), dim3(cps::kThreads),
+    if (!cuda_ok(c, cudaLaunchCooperativeKernel(grid_kernel_for(c), dim3(c->grid), dim3(cps::kThreads),
                                                 args, tile_smem_for(c->precision), c->stream), "cooperative launch"))
       return CPS_ERR_CUDA;
     if (!cuda_ok(c, cudaEventRecord(c->ev1, c->stream), "event")) return CPS_ERR_CUDA;
@@ -605,13 +632,17 @@ cps_status cps_create(const cps_desc* d, cps_ctx** out) {
 
   // Persistent grid: co-resident CTAs, at most one per tile of the design.
   int per_sm = 0, sms = 0;
-  if (!allow_smem(c, grid_kernel_for(d->precision), tile_smem_for(d->precision)) ||
-      !allow_smem(c, grid_kernel_for(d->precision, true), tile_smem_for(d->precision)) ||
-      !allow_smem(c, grid_kernel_for(d->precision, false, true), tile_smem_for(d->precision)) ||
-      !cuda_ok(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, grid_kernel_for(d->precision),
-                                                                cps::kThreads, tile_smem_for(d->precision)),
-               "occupancy") ||
-      !cuda_ok(c, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, d->device), "attribute"))
+  for (int k = 0; k < kGridKernels; ++k) {
+    // the kernels are interchangeable within a design, so the grid is what all of them allow
+    const void* fn = grid_kernel_of(d->precision, k);
+    int n = 0;
+    if (!allow_smem(c, fn, tile_smem_for(d->precision)) ||
+        !cuda_ok(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, cps::kThreads, tile_smem_for(d->precision)),
+                 "occupancy"))
+      return bail(CPS_ERR_CUDA);
+    per_sm = k == 0 ? n : std::min(per_sm, n);
+  }
+  if (!cuda_ok(c, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, d->device), "attribute"))
     return bail(CPS_ERR_CUDA);
   if (per_sm < 1) return bail(fail(c, CPS_ERR_CUDA, "persistent kernel does not fit on an SM"));
   const int tiles = ((d->M - 1 + cps::kTileI - 1) / cps::kTileI) * ((d->N - 1 + cps::kTileJ - 1) / cps::kTileJ);
@@ -892,10 +923,11 @@ cps_status cps_batch_solve(cps_ctx* const* ctxs, int n, const double* inletVeloc
   std::string err;
   BatchWorkspace* ws = batch_workspace(c0->device, (size_t)n, err);
   if (!ws) return fail(c0, CPS_ERR_OOM, err);
-  // The batch kernels carry the pseudo-transient term and the CFL controllers
-  // only when a design of the batch has them on (a separate instantiation:
-  // compiled in, they slow every batched outer iteration by a quarter).
-  bool pseudo = false;
+  // The batch kernels carry the options (the pseudo-transient term and the CFL
+  // controllers among them) only when a design of the batch has one on (a
+  // separate instantiation: compiled in, they slow every batched outer
+  // iteration by a quarter).
+  bool options = false;
   for (int k = 0; k < n; ++k) {
     cps_ctx* c = ctxs[k];
     set_step_inputs(c, inletVelocity ? inletVelocity[k] : c->view.Uin);
@@ -909,7 +941,7 @@ cps_status cps_batch_solve(cps_ctx* const* ctxs, int n, const double* inletVeloc
     it.hist = c->dhist;
     it.hist_cap = kHistChunk;
     it.iter0 = c->iter;
-    pseudo = pseudo || c->view.pseudo != 0;
+    options = options || has_options(c->view);
   }
   std::vector<int> ord(n);
   std::iota(ord.begin(), ord.end(), 0);
@@ -929,8 +961,8 @@ cps_status cps_batch_solve(cps_ctx* const* ctxs, int n, const double* inletVeloc
     // Groups sized to their designs, packed into waves (first fit, largest
     // first); one cooperative launch per wave, all CTAs of a wave co-resident.
     const void* wk = c0->precision == CPS_MIXED
-                         ? (pseudo ? (const void*)cps_wave_kernel<float, true> : (const void*)cps_wave_kernel<float, false>)
-                         : (pseudo ? (const void*)cps_wave_kernel<double, true> : (const void*)cps_wave_kernel<double, false>);
+                         ? (options ? (const void*)cps_wave_kernel<float, true> : (const void*)cps_wave_kernel<float, false>)
+                         : (options ? (const void*)cps_wave_kernel<double, true> : (const void*)cps_wave_kernel<double, false>);
     int per_sm = 0, sms = 0;
     const size_t tsm = tile_smem_for(c0->precision);
     if (!allow_smem(c0, wk, tsm) ||
@@ -990,8 +1022,8 @@ cps_status cps_batch_solve(cps_ctx* const* ctxs, int n, const double* inletVeloc
   } else if (opts->group_ctas > 0) {
     // Groups of CTAs in one cooperative launch (all CTAs co-resident).
     const void* gk = c0->precision == CPS_MIXED
-                         ? (pseudo ? (const void*)cps_group_kernel<float, true> : (const void*)cps_group_kernel<float, false>)
-                         : (pseudo ? (const void*)cps_group_kernel<double, true> : (const void*)cps_group_kernel<double, false>);
+                         ? (options ? (const void*)cps_group_kernel<float, true> : (const void*)cps_group_kernel<float, false>)
+                         : (options ? (const void*)cps_group_kernel<double, true> : (const void*)cps_group_kernel<double, false>);
     int per_sm = 0, sms = 0;
     const size_t tsm = tile_smem_for(c0->precision);
     if (!allow_smem(c0, gk, tsm) ||
@@ -1020,8 +1052,8 @@ cps_status cps_batch_solve(cps_ctx* const* ctxs, int n, const double* inletVeloc
   } else {
   using KernFn = void (*)(const cps::BatchItem*, const int*, int, int*, cps::BatchResult*);
   KernFn kern = c0->precision == CPS_MIXED
-                    ? (pseudo ? (KernFn)cps_cluster_kernel<float, true> : (KernFn)cps_cluster_kernel<float, false>)
-                    : (pseudo ? (KernFn)cps_cluster_kernel<double, true> : (KernFn)cps_cluster_kernel<double, false>);
+                    ? (options ? (KernFn)cps_cluster_kernel<float, true> : (KernFn)cps_cluster_kernel<float, false>)
+                    : (options ? (KernFn)cps_cluster_kernel<double, true> : (KernFn)cps_cluster_kernel<double, false>);
   if (cl > 8 &&
       !cuda_ok(c0, cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1), "attr"))
     return CPS_ERR_CUDA;

@@ -1,0 +1,3 @@
+#include "cps_kernels.cuh"
+
+CPS_BATCH_OPTION_KERNELS(, double)

@@ -84,15 +84,6 @@ constexpr int kRedSlots = 4;    // ring of reduction slots (grid group)
 #define CPS_MIN_BLOCKS 2
 #endif
 constexpr int kStageDepth = 3;  // tiles whose shared-memory copies are in flight at once
-// PCG with the CTA's unknowns in shared memory for designs of up to
-// SmemTiles<T> tiles per CTA (0: the global-memory PCG there).
-#ifndef CPS_SMEM_PCG
-#define CPS_SMEM_PCG 1
-#endif
-#ifndef CPS_RESIDENT_TILES
-#define CPS_RESIDENT_TILES 2
-#endif
-constexpr int kResidentTiles = CPS_RESIDENT_TILES;  // register-resident PCG up to this many tiles per CTA
 constexpr unsigned long long kBarrierTimeoutNs = 2000000000ull;  // 2 s
 constexpr unsigned long long kTmaTimeoutNs = 1000000000ull;      // a tile copy that has not landed after 1 s
 constexpr unsigned long long kTmaDrainNs = 10000000ull;          // then wait up to 10 ms for the copies in flight
@@ -115,6 +106,14 @@ enum TmaMap : int {
   kTmCV_B, kTmBV_B = kTmCV_B + 5, kTmXV0_B, kTmXV1_B,
   kTmCount
 };
+
+// What a kernel instantiation carries: the PCG forms its designs may need and
+// the options off the default path (single-reduction PCG, explicit momentum,
+// TMA-staged sweeps).  Each form inlined beside the others takes registers
+// from every phase (all forms and options in one kernel: 165 bytes of spills,
+// late outer iterations 5 % slower), so the host launches the least that a
+// design needs.
+enum Carries : int { kFew = 1, kMany = 2, kLarge = 4, kForms = 7, kOptions = 8, kAll = 15 };
 
 enum DeviceStatus : int { kStatusOk = 0, kStatusTimeout = 1, kStatusDiverged = 2 };
 
@@ -194,7 +193,6 @@ struct PseudoRun {
 // reductions, so every thread holds the same values).
 struct SweepHint {
   int kU, kV;
-  int kP;  // the PCG's count (iterations after the first) of the last outer iteration
 };
 
 template <typename T> __device__ __forceinline__ const Inner<T>& inner(const DesignView& d);
@@ -287,6 +285,12 @@ __device__ __forceinline__ double div_rn(double a, double b, double y) {
   return (__double2hiint(v) & 0x7ff00000) == 0x7ff00000 ? q : v;
 }
 __device__ __forceinline__ double div_rn(double a, double b) { return div_rn(a, b, recip(b)); }
+// a / b for a value that every thread of the group holds: any operands, the
+// branch taken by all threads alike.
+__device__ __forceinline__ double div_uniform(double a, double b) {
+  const unsigned ea = ((unsigned)__double2hiint(a) >> 20) & 0x7ffu, eb = ((unsigned)__double2hiint(b) >> 20) & 0x7ffu;
+  return (ea - 523u <= 1000u && eb - 523u <= 1000u) ? div_rn(a, b) : a / b;  // both within 2^+-500
+}
 
 // ---------------------------------------------------------------------------
 // Pseudo-transient term and CFL controllers
@@ -1296,386 +1300,481 @@ __device__ __forceinline__ double sweep_point(const DesignView& d, int i, int j,
   return r * r;
 }
 
-// ---------------------------------------------------------------------------
-// PCG as the reference runs it (pressure_solver.cpp:121-184): two grid-wide
-// reductions per iteration (p.Ap, then |r|^2 and r.z).  Phase P1 forms
-// p = z + beta p on the fly for the 5-point stencil and Ap; phase P2 updates
-// x, r, z.  Both load straight from global memory, every load of a point
-// issued before its first store so that the loads overlap (staging these two
-// light phases through shared memory measured slower on B200).  Returns the
-// reference's iteration count, or -1 if a wait failed.
-// ---------------------------------------------------------------------------
+// x = 0 for phase D, when the PCG stops before its first update.
 template <typename T, class Group>
-__device__ int pcg_two_reductions(const DesignView& d, Group& g, double* smem, double rz0, double pAp0) {
+__device__ __forceinline__ int no_update(const DesignView& d, Group& g) {
+  const Inner<T>& w = inner<T>(d);
+  for_each_point(d, g.rank, g.nblk, [&](int i, int j) {
+    if (j <= d.N - 2) w.px[(size_t)i * d.P + j] = (T)0;
+  });
+  return g.sync() ? 0 : -1;
+}
+
+// r - alpha A p and z = r / diag of one unknown, in the storage type.
+template <typename T>
+__device__ __forceinline__ T residual_of(T r, double alpha, T ap) { return (T)((double)r - alpha * (double)ap); }
+template <typename T>
+__device__ __forceinline__ T precond_of(T r, T dg) {
+  const double dgd = (double)dg;
+  return (T)((fabs(dgd) > 1e-20) ? div_rn((double)r, dgd) : (double)r);
+}
+
+// Iteration 0 (x0 = 0; p0 = z0, A p0 and p0.A p0 come from phase C): x, and
+// |r|^2 and r.z in s2.  Late in a solve it is the only one, so r and z are
+// stored only for the form that reads them back (Store); pcg_tiles forms them
+// again from the same planes.
+template <typename T, bool Store, class Group>
+__device__ __forceinline__ bool pcg_first(const DesignView& d, Group& g, double* smem, double alpha, double (&s2)[2]) {
+  const Inner<T>& w = inner<T>(d);
+  const int N = d.N, P = d.P;
+  for_each_point(d, g.rank, g.nblk, [&](int i, int j) {
+    if (j > N - 2) return;
+    const size_t o = (size_t)i * P + j;
+    const T pc = w.pp0[o], ro = w.pr[o], ap = w.pAp[o], dg = w.pdiag[o];
+    w.px[o] = (T)(0.0 + alpha * (double)pc);
+    const T rt = residual_of(ro, alpha, ap);
+    const T z = precond_of(rt, dg);
+    if (Store) {
+      w.pr[o] = rt;
+      w.pz[o] = z;
+    }
+    const double r = (double)rt;
+    s2[0] += r * r;
+    s2[1] += r * (double)z;
+  });
+  return g.template sync_reduce<2, 0u>(s2, smem);
+}
+
+// Iterations 1, 2, ... from global memory; rz = r.z, beta of iteration 1.
+template <typename T, class Group>
+__device__ __forceinline__ int pcg_global(const DesignView& d, Group& g, double* smem, double rz, double beta) {
   const Inner<T>& w = inner<T>(d);
   const int M = d.M, N = d.N, P = d.P;
-  double rz = rz0, beta = 0.0;
-  int it = 0;
+  int it = 1;
   for (; it < d.maxPIter; ++it) {
     const T* pold = (it & 1) ? w.pp0 : w.pp1;  // p_{it-1}
     T* pcur = (it & 1) ? w.pp1 : w.pp0;        // p_it
     const double bt = beta;
-    double s1[1] = {pAp0};  // iteration 0's p = z, A p and p.Ap come from phase C
-    if (it > 0) {
-      s1[0] = 0.0;
-      for_each_point(d, g.rank, g.nblk, [&](int i, int j) {
-        if (j > N - 2) return;
-        const size_t o = (size_t)i * P + j;
-        // p_k at (i, j) and its unknown neighbours: p = z + beta p (pressure_solver.cpp:181)
-        auto pk = [&](size_t q) -> double { return (double)(T)((double)w.pz[q] + bt * (double)pold[q]); };
-        const double pc0 = pk(o);
-        double Ap = 0.0;
-        if (i > 1) Ap += -(double)w.cy[o - P] * pk(o - P);
-        if (j > 1) Ap += -(double)w.cx[o - 1] * pk(o - 1);
-        Ap += (double)w.pdiag[o] * pc0;
-        if (j + 1 <= N - 2) Ap += -(double)w.cx[o] * pk(o + 1);
-        if (i < M - 1) Ap += -(double)w.cy[o] * pk(o + P);
-        pcur[o] = (T)pc0;
-        const T apt = (T)Ap;
-        w.pAp[o] = apt;
-        s1[0] += pc0 * (double)apt;
-      });
-      if (!g.template sync_reduce<1, 0u>(s1, smem)) return -1;
-    }
+    double s1[1] = {0.0};
+    for_each_point(d, g.rank, g.nblk, [&](int i, int j) {
+      if (j > N - 2) return;
+      const size_t o = (size_t)i * P + j;
+      // p_k at (i, j) and its unknown neighbours: p = z + beta p (pressure_solver.cpp:181)
+      auto pk = [&](size_t q) -> double { return (double)(T)((double)w.pz[q] + bt * (double)pold[q]); };
+      const double pc0 = pk(o);
+      double Ap = 0.0;
+      if (i > 1) Ap += -(double)w.cy[o - P] * pk(o - P);
+      if (j > 1) Ap += -(double)w.cx[o - 1] * pk(o - 1);
+      Ap += (double)w.pdiag[o] * pc0;
+      if (j + 1 <= N - 2) Ap += -(double)w.cx[o] * pk(o + 1);
+      if (i < M - 1) Ap += -(double)w.cy[o] * pk(o + P);
+      pcur[o] = (T)pc0;
+      const T apt = (T)Ap;
+      w.pAp[o] = apt;
+      s1[0] += pc0 * (double)apt;
+    });
+    if (!g.template sync_reduce<1, 0u>(s1, smem)) return -1;
     const double pAp = s1[0];
     if (fabs(pAp) < 1e-20) break;
-    const double alpha = rz / pAp;
+    const double alpha = div_uniform(rz, pAp);
     double s2[2] = {0.0, 0.0};  // |r|^2, r.z
     for_each_point(d, g.rank, g.nblk, [&](int i, int j) {
       if (j > N - 2) return;
       const size_t o = (size_t)i * P + j;
       const T xo = w.px[o], pc = pcur[o], ro = w.pr[o], ap = w.pAp[o], dgo = w.pdiag[o];
       w.px[o] = (T)((double)xo + alpha * (double)pc);
-      const T rt = (T)((double)ro - alpha * (double)ap);
+      const T rt = residual_of(ro, alpha, ap);
       w.pr[o] = rt;
       const double r = (double)rt;
       s2[0] += r * r;
-      const double dg = (double)dgo;
-      const T z = (T)((fabs(dg) > 1e-20) ? div_rn(r, dg) : r);
+      const T z = precond_of(rt, dgo);
       w.pz[o] = z;
       s2[1] += r * (double)z;
     });
     if (!g.template sync_reduce<2, 0u>(s2, smem)) return -1;
     if (s2[0] < d.pStop) break;
-    const double rzPrev = rz;
+    beta = div_uniform(s2[1], rz);
     rz = s2[1];
-    beta = rz / rzPrev;
   }
   return it;
 }
 
 // ---------------------------------------------------------------------------
-// The same PCG for groups in which a thread owns at most R unknowns (every
-// CTA has at most R tiles): each thread keeps its unknowns' x, r, z, p, Ap,
-// diagonal and face conductances in registers for the whole solve, so P2
-// reads no memory (it stores x for phase D and z for the neighbours) and P1
-// loads only the neighbours' z and p_{k-1} (and stores p_k for them).  The
-// arithmetic, the points' order and so every sum are those of
-// pcg_two_reductions.
-// ---------------------------------------------------------------------------
-template <typename T, int R, class Group>
-__device__ int pcg_resident(const DesignView& d, Group& g, double* smem, double rz0, double pAp0) {
-  const Inner<T>& w = inner<T>(d);
-  const int M = d.M, N = d.N, P = d.P;
-  const int tilesJ = (N - 1 + kTileJ - 1) / kTileJ;
-  const int tilesI = (M - 1 + kTileI - 1) / kTileI;
-  const int nt = tilesI * tilesJ;
-  const int ty = (int)threadIdx.x / kTileJ, tx = (int)threadIdx.x % kTileJ;
-  bool on[R];
-  int ii[R], jj[R];
-  size_t oo[R];
-  T x[R], r[R], z[R], p[R], ap[R], dg[R], cE[R], cW[R], cN[R], cS[R];
-#pragma unroll
-  for (int u = 0; u < R; ++u) {
-    const int t = (int)g.rank + u * (int)g.nblk;
-    ii[u] = 1 + (t / tilesJ) * kTileI + ty;
-    jj[u] = 1 + (t % tilesJ) * kTileJ + tx;
-    on[u] = t < nt && ii[u] <= M - 1 && jj[u] <= N - 2;
-    oo[u] = on[u] ? (size_t)ii[u] * P + jj[u] : 0;
-    x[u] = r[u] = z[u] = p[u] = ap[u] = dg[u] = cE[u] = cW[u] = cN[u] = cS[u] = (T)0;
-    if (on[u]) {
-      const size_t o = oo[u];
-      x[u] = w.px[o];
-      r[u] = w.pr[o];
-      z[u] = w.pz[o];
-      p[u] = w.pp0[o];
-      ap[u] = w.pAp[o];
-      dg[u] = w.pdiag[o];
-      cE[u] = w.cx[o];
-      cN[u] = w.cy[o];
-      if (jj[u] > 1) cW[u] = w.cx[o - 1];
-      if (ii[u] > 1) cS[u] = w.cy[o - P];
-    }
-  }
-  double rz = rz0, beta = 0.0;
-  int it = 0;
-  for (; it < d.maxPIter; ++it) {
-    const T* pold = (it & 1) ? w.pp0 : w.pp1;  // p_{it-1}
-    T* pcur = (it & 1) ? w.pp1 : w.pp0;        // p_it
-    const double bt = beta;
-    double s1[1] = {pAp0};  // iteration 0's p = z, A p and p.Ap come from phase C
-    if (it > 0) {
-      s1[0] = 0.0;
-      T zn[R][4], pn[R][4];  // z and p_{k-1} at the S, W, E, N neighbours
-#pragma unroll
-      for (int u = 0; u < R; ++u) {
-#pragma unroll
-        for (int q = 0; q < 4; ++q) zn[u][q] = pn[u][q] = (T)0;
-        if (on[u]) {
-          const size_t o = oo[u];
-          if (ii[u] > 1) { zn[u][0] = w.pz[o - P]; pn[u][0] = pold[o - P]; }
-          if (jj[u] > 1) { zn[u][1] = w.pz[o - 1]; pn[u][1] = pold[o - 1]; }
-          if (jj[u] + 1 <= N - 2) { zn[u][2] = w.pz[o + 1]; pn[u][2] = pold[o + 1]; }
-          if (ii[u] < M - 1) { zn[u][3] = w.pz[o + P]; pn[u][3] = pold[o + P]; }
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < R; ++u) {
-        if (!on[u]) continue;
-        const int i = ii[u], j = jj[u];
-        // p = z + beta p (pressure_solver.cpp:181) at the point and its unknown neighbours
-        auto pk = [&](T zq, T pq) -> double { return (double)(T)((double)zq + bt * (double)pq); };
-        const double pc0 = pk(z[u], p[u]);
-        double Ap = 0.0;
-        if (i > 1) Ap += -(double)cS[u] * pk(zn[u][0], pn[u][0]);
-        if (j > 1) Ap += -(double)cW[u] * pk(zn[u][1], pn[u][1]);
-        Ap += (double)dg[u] * pc0;
-        if (j + 1 <= N - 2) Ap += -(double)cE[u] * pk(zn[u][2], pn[u][2]);
-        if (i < M - 1) Ap += -(double)cN[u] * pk(zn[u][3], pn[u][3]);
-        p[u] = (T)pc0;
-        pcur[oo[u]] = p[u];
-        ap[u] = (T)Ap;
-        s1[0] += pc0 * (double)ap[u];
-      }
-      if (!g.template sync_reduce<1, 0u>(s1, smem)) return -1;
-    }
-    const double pAp = s1[0];
-    if (fabs(pAp) < 1e-20) break;
-    const double alpha = rz / pAp;
-    double s2[2] = {0.0, 0.0};  // |r|^2, r.z
-#pragma unroll
-    for (int u = 0; u < R; ++u) {
-      if (!on[u]) continue;
-      x[u] = (T)((double)x[u] + alpha * (double)p[u]);
-      w.px[oo[u]] = x[u];
-      const T rt = (T)((double)r[u] - alpha * (double)ap[u]);
-      r[u] = rt;
-      const double rr = (double)rt;
-      s2[0] += rr * rr;
-      const double dgd = (double)dg[u];
-      const T zz = (T)((fabs(dgd) > 1e-20) ? div_rn(rr, dgd) : rr);
-      z[u] = zz;
-      w.pz[oo[u]] = zz;
-      s2[1] += rr * (double)zz;
-    }
-    if (!g.template sync_reduce<2, 0u>(s2, smem)) return -1;
-    if (s2[0] < d.pStop) break;
-    const double rzPrev = rz;
-    rz = s2[1];
-    beta = rz / rzPrev;
-  }
-  return it;
-}
-
-// ---------------------------------------------------------------------------
-// The same PCG with the CTA's unknowns in shared memory, for groups in which a
-// CTA owns more tiles than fit in registers but at most R (SmemTiles<T>): r,
-// z, p, Ap and the east/north face conductances of every point of the CTA's
-// tiles (mixed: also the diagonal and x) are loaded once, and each PCG
-// iteration then reads global memory only for the neighbours that lie in
-// another tile (the ring around each tile: z and p_{k-1}, copied with
-// cp.async for all tiles at once, each thread into halo slots only it reads).
-//   P1 forms p_k = z + beta p_{k-1} once at each of the CTA's points, in
-//   place, then (after a CTA barrier) Ap from it, and from z and p_{k-1} at the
-//   halo with the same expression; P2 updates x, r, z and stores p_k and z to
-//   global memory for the other tiles.
-// FP64 forms the diagonal from the four conductances the way phase C did (the
-// stored conductances are phase C's summands, added in its order), and keeps x
-// at the thread's points in registers (x + alpha p, one rounding, as P2
-// forms it), storing it every iteration so that the last store precedes the
-// last grid barrier and phase D reads the final x.  The points, their order
-// and every sum are those of pcg_two_reductions, so the iterates are the same
-// bits.
+// The same iterations for groups whose CTAs own at most R tiles each
+// (PcgTiles): x, r and A p of a thread's points stay in registers, p with a
+// one-point ring, z, the conductances, the diagonal and its reciprocal in
+// shared memory, so that an iteration touches global memory only for the z of
+// the points at a tile's edge, which the neighbouring tiles read (they keep p
+// at their ring and form p = z + beta p there themselves, with the owner's
+// expression).
+//   P1: p = z + beta p at the CTA's points and ring, a CTA barrier, A p;
+//   P2: x, r, z, and z to global memory at the tiles' edges.
+// Values beyond the unknowns are held as zeros, so the stencil has no
+// conditions.  x goes to global memory in the last iteration the cap allows,
+// before the reduction whose barrier phase D relies on; a stop before that
+// stores it and waits once more.  The points, their order and every sum are
+// those of pcg_global, so the iterates are the same bits.
+//
+// What it replaced kept r, z, p, A p in shared memory for 3..7 tiles per CTA
+// (p and z of every point to global memory, tile indices divided out per tile
+// and pass) and read 8 neighbour values per point from L2 for 1..2 tiles.
+// B200, us per CG iteration, FP64 / mixed: 1000 x 500 (7 tiles) 14.1 -> 8.2 /
+// 15.7 -> 8.9; 512 x 256 (2 tiles) 6.1 -> 5.7 / 6.9 -> 5.9.  What is left is
+// the two grid reductions (4.4) and about 30 shared-memory and FP64 operations
+// per point.
 // ---------------------------------------------------------------------------
 constexpr int kHalo = 2 * kTileJ + 2 * kTileI;  // a tile's south row, north row, west column, east column
 
+// Place of ring point q (south row, north row, west column, east column) in a
+// tile's p with its ring, and its position relative to the tile's first point.
+__device__ __forceinline__ int ring_place(int q, int& a, int& b) {
+  if (q < kTileJ) { a = -1; b = q; }
+  else if (q < 2 * kTileJ) { a = kTileI; b = q - kTileJ; }
+  else if (q < 2 * kTileJ + kTileI) { a = q - 2 * kTileJ; b = -1; }
+  else { a = q - 2 * kTileJ - kTileI; b = kTileJ; }
+  return (a + 1) * (kTileJ + 2) + b + 1;
+}
+
+// Tiles per CTA the two builds of the form hold: few (small designs) and what
+// two CTAs per SM leave of shared memory.
+constexpr int kFewTiles = 2;
 template <typename T>
-struct SmemTiles {
+struct PcgTileCount {
   static constexpr int value = sizeof(T) == 8 ? 7 : 12;
 };
 
 template <typename T, int R>
-struct PcgSmem {
-  static constexpr int kM = sizeof(T) == 4 ? R : 1;  // arrays the mixed mode keeps in addition
-  T r[R][kThreads], z[R][kThreads], p[R][kThreads], ap[R][kThreads], cE[R][kThreads], cN[R][kThreads];
-  T dg[kM][kThreads], x[kM][kThreads];
-  T zH[R][kHalo], pH[R][kHalo];      // z and p_{k-1} at the neighbours in other tiles
-  T cWH[R][kTileI], cSH[R][kTileJ];  // the west / south conductances at the tile's west / south edge
+struct PcgTiles {
+  static constexpr int kPW = kTileJ + 2, kPN = (kTileI + 2) * kPW;  // p and its ring
+  static constexpr int kEW = kTileJ + 1, kEN = kTileI * kEW;        // east conductances from column -1
+  static constexpr int kNN = (kTileI + 1) * kTileJ;                 // north conductances from row -1
+  double inv[R][kThreads];  // recip(diagonal); 0 where the preconditioner leaves r
+  T p[R][kPN], cE[R][kEN], cN[R][kNN], dg[R][kThreads], z[R][kThreads];
+  int origin[R];  // element offset of the tile's first point
 };
 
+// alpha0: iteration 0's alpha (r and z of iteration 1 are formed from phase C's planes).
 template <typename T, int R, class Group>
-__device__ int pcg_smem(const DesignView& d, Group& g, double* smem, char* tbuf, double rz0, double pAp0) {
-  constexpr bool kMixed = sizeof(T) == 4;
-  PcgSmem<T, R>& S = *reinterpret_cast<PcgSmem<T, R>*>(tbuf);
+__device__ __forceinline__ int pcg_tiles(const DesignView& d, Group& g, double* smem, char* tbuf, double alpha0,
+                                         double rz, double beta) {
+  using Sm = PcgTiles<T, R>;
+  constexpr int kPW = Sm::kPW, kEW = Sm::kEW;
+  constexpr int kHM = (R * kHalo + kThreads - 1) / kThreads;  // ring points a thread looks after
+  Sm& S = *reinterpret_cast<Sm*>(tbuf);
   const Inner<T>& w = inner<T>(d);
   const int M = d.M, N = d.N, P = d.P;
   const int tilesJ = (N - 1 + kTileJ - 1) / kTileJ;
-  const int tilesI = (M - 1 + kTileI - 1) / kTileI;
-  const int nt = tilesI * tilesJ;
-  const int ty = (int)threadIdx.x / kTileJ, tx = (int)threadIdx.x % kTileJ, th = threadIdx.x;
+  const int nt = tilesJ * ((M - 1 + kTileI - 1) / kTileI);
+  const int th = threadIdx.x, ty = th / kTileJ, tx = th % kTileJ;
   const int nk = (int)g.rank < nt ? (nt - 1 - (int)g.rank) / (int)g.nblk + 1 : 0;  // this CTA's tiles
-  T* const pg = w.pp0;  // p_k in global memory for the other tiles (read by P1 of the next iteration)
-  // the thread's point in its k-th tile; true: a pressure unknown
-  auto point = [&](int k, int& i, int& j) {
-    const int t = (int)g.rank + k * (int)g.nblk;
-    i = 1 + (t / tilesJ) * kTileI + ty;
-    j = 1 + (t % tilesJ) * kTileJ + tx;
-    return i <= M - 1 && j <= N - 2;
-  };
-  // the west / south conductances of the thread's point in tile k
-  auto cW = [&](int k, int j) -> T { return j > 1 ? (tx > 0 ? S.cE[k][th - 1] : S.cWH[k][ty]) : (T)0; };
-  auto cS = [&](int k, int i) -> T { return i > 1 ? (ty > 0 ? S.cN[k][th - kTileJ] : S.cSH[k][tx]) : (T)0; };
-  // the diagonal (pressure_solver.cpp:703-706 as phase C evaluates it)
-  auto diag = [&](int k, int i, int j) -> double {
-    if constexpr (kMixed) {
-      return (double)S.dg[k][th];
-    } else {
-      double aP = (double)S.cE[k][th] + (double)cW(k, j) + (double)S.cN[k][th] + (double)cS(k, i);
-      if (aP < 1e-20) aP = 1.0;
-      return aP;
-    }
-  };
-  // state from phase C: r0, z0, p0 = z0, A p0 and the conductances
-  for (int k = 0; k < nk; ++k) {
-    int i, j;
-    if (!point(k, i, j)) continue;
-    const size_t o = (size_t)i * P + j;
-    cp_async_elem(&S.r[k][th], w.pr + o);
-    cp_async_elem(&S.z[k][th], w.pz + o);
-    cp_async_elem(&S.p[k][th], w.pp0 + o);
-    cp_async_elem(&S.ap[k][th], w.pAp + o);
-    cp_async_elem(&S.cE[k][th], w.cx + o);
-    cp_async_elem(&S.cN[k][th], w.cy + o);
-    if constexpr (kMixed) {
-      cp_async_elem(&S.dg[k][th], w.pdiag + o);
-      S.x[k][th] = (T)0;  // phase C's x0
-    }
-    if (tx == 0 && j > 1) cp_async_elem(&S.cWH[k][ty], w.cx + o - 1);
-    if (ty == 0 && i > 1) cp_async_elem(&S.cSH[k][tx], w.cy + o - P);
-  }
-  cp_async_commit();
-  cp_async_wait<0>();
-  __syncthreads();
-  double rz = rz0, beta = 0.0;
-  double xr[R];  // FP64: x at the thread's points (phase C's x0 = 0)
+  const int lo = ty * P + tx, ip = (ty + 1) * kPW + tx + 1, ie = ty * kEW + tx + 1, in = (ty + 1) * kTileJ + tx;
+  const bool edge = ty == 0 || ty == kTileI - 1 || tx == 0 || tx == kTileJ - 1;
+  unsigned on = 0;  // bit k: the thread's point in tile k is a pressure unknown
+  T x[R], r[R], ap[R];
 #pragma unroll
-  for (int k = 0; k < R; ++k) xr[k] = 0.0;
-  int it = 0;
-  for (; it < d.maxPIter; ++it) {
-    const double bt = beta;
-    // p = z + beta p (pressure_solver.cpp:181)
-    auto pk = [&](T zq, T pq) -> double { return (double)(T)((double)zq + bt * (double)pq); };
-    double s1[1] = {pAp0};  // iteration 0's p = z, A p and p.Ap come from phase C
-    if (it > 0) {
-      s1[0] = 0.0;
-      // the neighbours in other tiles, every tile's at once
-      for (int k = 0; k < nk; ++k) {
-        int i, j;
-        if (!point(k, i, j)) continue;
-        const size_t o = (size_t)i * P + j;
-        if (ty == 0 && i > 1) {
-          cp_async_elem(&S.zH[k][tx], w.pz + o - P);
-          cp_async_elem(&S.pH[k][tx], pg + o - P);
-        }
-        if (ty == kTileI - 1 && i < M - 1) {
-          cp_async_elem(&S.zH[k][kTileJ + tx], w.pz + o + P);
-          cp_async_elem(&S.pH[k][kTileJ + tx], pg + o + P);
-        }
-        if (tx == 0 && j > 1) {
-          cp_async_elem(&S.zH[k][2 * kTileJ + ty], w.pz + o - 1);
-          cp_async_elem(&S.pH[k][2 * kTileJ + ty], pg + o - 1);
-        }
-        if (tx == kTileJ - 1 && j + 1 <= N - 2) {
-          cp_async_elem(&S.zH[k][2 * kTileJ + kTileI + ty], w.pz + o + 1);
-          cp_async_elem(&S.pH[k][2 * kTileJ + kTileI + ty], pg + o + 1);
-        }
-      }
-      cp_async_commit();
-      // p_it at the CTA's own points, formed once in place (the stencil below
-      // and P2 read it; the value of forming it at every use)
-      for (int k = 0; k < nk; ++k) {
-        int i, j;
-        if (!point(k, i, j)) continue;
-        S.p[k][th] = (T)pk(S.z[k][th], S.p[k][th]);
-      }
-      cp_async_wait<0>();  // each thread reads only the halo slots it copied
-      __syncthreads();     // and its tile's p_it after every thread has formed its own
-      for (int k = 0; k < nk; ++k) {
-        int i, j;
-        if (!point(k, i, j)) continue;
-        const double pc0 = (double)S.p[k][th];
-        double Ap = 0.0;
-        if (i > 1) {
-          if (ty > 0) Ap += -(double)S.cN[k][th - kTileJ] * (double)S.p[k][th - kTileJ];
-          else Ap += -(double)S.cSH[k][tx] * pk(S.zH[k][tx], S.pH[k][tx]);
-        }
-        if (j > 1) {
-          if (tx > 0) Ap += -(double)S.cE[k][th - 1] * (double)S.p[k][th - 1];
-          else Ap += -(double)S.cWH[k][ty] * pk(S.zH[k][2 * kTileJ + ty], S.pH[k][2 * kTileJ + ty]);
-        }
-        Ap += diag(k, i, j) * pc0;
-        if (j + 1 <= N - 2) {
-          const int q = 2 * kTileJ + kTileI + ty;
-          Ap += -(double)S.cE[k][th] * (tx < kTileJ - 1 ? (double)S.p[k][th + 1] : pk(S.zH[k][q], S.pH[k][q]));
-        }
-        if (i < M - 1) {
-          const int q = kTileJ + tx;
-          Ap += -(double)S.cN[k][th] *
-                (ty < kTileI - 1 ? (double)S.p[k][th + kTileJ] : pk(S.zH[k][q], S.pH[k][q]));
-        }
-        const T apt = (T)Ap;
-        S.ap[k][th] = apt;
-        s1[0] += pc0 * (double)apt;
-      }
-      if (!g.template sync_reduce<1, 0u>(s1, smem)) return -1;
+  for (int k = 0; k < R; ++k) {
+    x[k] = r[k] = (T)0;
+    if (k >= nk) continue;
+    const int t = (int)g.rank + k * (int)g.nblk;
+    const int i0 = 1 + (t / tilesJ) * kTileI, j0 = 1 + (t % tilesJ) * kTileJ, o0 = i0 * P + j0;
+    const bool mine = i0 + ty <= M - 1 && j0 + tx <= N - 2;
+    on |= mine ? 1u << k : 0u;
+    const int o = mine ? o0 + lo : P + 1;
+    const T ro = w.pr[o], apo = w.pAp[o], xo = w.px[o], pc = w.pp0[o], dgo = w.pdiag[o], ce = w.cx[o], cn = w.cy[o];
+    if (th == 0) S.origin[k] = o0;
+    if (mine) {
+      x[k] = xo;
+      r[k] = residual_of(ro, alpha0, apo);
     }
+    const double dgd = (double)dgo;
+    S.inv[k][th] = fabs(dgd) > 1e-20 ? recip(dgd) : 0.0;
+    S.z[k][th] = mine ? precond_of(r[k], dgo) : (T)0;
+    S.p[k][ip] = mine ? pc : (T)0;
+    S.dg[k][th] = dgo;
+    S.cE[k][ie] = mine ? ce : (T)0;
+    S.cN[k][in] = mine ? cn : (T)0;
+    if (tx == 0) S.cE[k][ie - 1] = (mine && j0 > 1) ? w.cx[o - 1] : (T)0;
+    if (ty == 0) S.cN[k][in - kTileJ] = (mine && i0 > 1) ? w.cy[o - P] : (T)0;
+  }
+  // the thread's ring points: element offset (-1: no unknown there) and place in S.p
+  int hoff[kHM], hdst[kHM];
+  T zh[kHM];
+  T* const sp = &S.p[0][0];
+#pragma unroll
+  for (int m = 0; m < kHM; ++m) {
+    hoff[m] = -1;
+    hdst[m] = 0;
+    zh[m] = (T)0;
+    const int e = th + m * kThreads;
+    if (e >= nk * kHalo) continue;
+    const int k = e / kHalo, q = e - k * kHalo, t = (int)g.rank + k * (int)g.nblk;
+    int a, b;
+    hdst[m] = k * Sm::kPN + ring_place(q, a, b);
+    const int i = 1 + (t / tilesJ) * kTileI + a, j = 1 + (t % tilesJ) * kTileJ + b;
+    T pc = (T)0;
+    if (i >= 1 && i <= M - 1 && j >= 1 && j <= N - 2) {
+      hoff[m] = i * P + j;
+      pc = w.pp0[hoff[m]];
+      zh[m] = precond_of(residual_of(w.pr[hoff[m]], alpha0, w.pAp[hoff[m]]), w.pdiag[hoff[m]]);
+    }
+    sp[hdst[m]] = pc;
+  }
+  __syncthreads();
+  bool stored = true;  // w.px holds x
+  int it = 1;
+  for (; it < d.maxPIter; ++it) {
+    // p = z + beta p (pressure_solver.cpp:181)
+    auto pk = [&](T zq, T pq) -> T { return (T)((double)zq + beta * (double)pq); };
+    if (it > 1) {
+      // z at the ring, written by the neighbours before the last reduction
+#pragma unroll
+      for (int m = 0; m < kHM; ++m)
+        if (hoff[m] >= 0) zh[m] = __ldcg(w.pz + hoff[m]);
+    }
+#pragma unroll
+    for (int k = 0; k < R; ++k) {
+      if (k >= nk) break;
+      S.p[k][ip] = pk(S.z[k][th], S.p[k][ip]);
+    }
+#pragma unroll
+    for (int m = 0; m < kHM; ++m)
+      if (hoff[m] >= 0) sp[hdst[m]] = pk(zh[m], sp[hdst[m]]);
+    __syncthreads();
+    double s1[1] = {0.0};
+#pragma unroll
+    for (int k = 0; k < R; ++k) {
+      if (k >= nk) break;
+      const T* q = &S.p[k][ip];
+      const double pc = (double)q[0];
+      double Ap = 0.0;
+      Ap += -(double)S.cN[k][in - kTileJ] * (double)q[-kPW];
+      Ap += -(double)S.cE[k][ie - 1] * (double)q[-1];
+      Ap += (double)S.dg[k][th] * pc;
+      Ap += -(double)S.cE[k][ie] * (double)q[1];
+      Ap += -(double)S.cN[k][in] * (double)q[kPW];
+      ap[k] = ((on >> k) & 1u) ? (T)Ap : (T)0;  // not an unknown: stays 0 throughout
+      s1[0] += pc * (double)ap[k];
+    }
+    if (!g.template sync_reduce<1, 0u>(s1, smem)) return -1;
     const double pAp = s1[0];
     if (fabs(pAp) < 1e-20) break;
-    const double alpha = rz / pAp;
+    const double alpha = div_uniform(rz, pAp);
+    stored = it + 1 == d.maxPIter;
     double s2[2] = {0.0, 0.0};  // |r|^2, r.z
 #pragma unroll
-    for (int k = 0; k < R; ++k) {  // unrolled: xr[k] stays in a register
+    for (int k = 0; k < R; ++k) {
       if (k >= nk) break;
-      int i, j;
-      if (!point(k, i, j)) continue;
-      const size_t o = (size_t)i * P + j;
-      const T pc = S.p[k][th];  // p_it (P1 formed it in place; iteration 0: p0 = z0)
-      pg[o] = pc;
-      if constexpr (kMixed) {
-        const T xn = (T)((double)S.x[k][th] + alpha * (double)pc);
-        S.x[k][th] = xn;
-        w.px[o] = xn;
-      } else {
-        xr[k] = xr[k] + alpha * (double)pc;  // x += alpha p (pressure_solver.cpp:164)
-        w.px[o] = xr[k];
+      x[k] = (T)((double)x[k] + alpha * (double)S.p[k][ip]);
+      r[k] = residual_of(r[k], alpha, ap[k]);
+      const double rr = (double)r[k], y = S.inv[k][th];
+      s2[0] += rr * rr;
+      const T z = (T)(__double2hiint(y) != 0 ? div_rn(rr, (double)S.dg[k][th], y) : rr);
+      S.z[k][th] = z;
+      s2[1] += rr * (double)z;
+      if (((on >> k) & 1u) && (edge || stored)) {
+        const int o = S.origin[k] + lo;
+        if (edge) w.pz[o] = z;
+        if (stored) w.px[o] = x[k];
       }
-      const T rt = (T)((double)S.r[k][th] - alpha * (double)S.ap[k][th]);
-      S.r[k][th] = rt;
-      const double r = (double)rt;
-      s2[0] += r * r;
-      const double dgd = diag(k, i, j);
-      const T zt = (T)((fabs(dgd) > 1e-20) ? div_rn(r, dgd) : r);
-      S.z[k][th] = zt;
-      w.pz[o] = zt;
-      s2[1] += r * (double)zt;
     }
     if (!g.template sync_reduce<2, 0u>(s2, smem)) return -1;
     if (s2[0] < d.pStop) break;
-    const double rzPrev = rz;
+    beta = div_uniform(s2[1], rz);
     rz = s2[1];
-    beta = rz / rzPrev;
+  }
+  if (!stored) {
+#pragma unroll
+    for (int k = 0; k < R; ++k)
+      if ((on >> k) & 1u) w.px[S.origin[k] + lo] = x[k];
+    if (!g.sync()) return -1;
   }
   return it;
+}
+
+// ---------------------------------------------------------------------------
+// The same for groups whose CTAs own more tiles than that, up to R: p with its
+// ring stays in shared memory and the other vectors stream from L2, four
+// tiles' loads before the first of their stores.  Against pcg_global, which
+// this replaces there, an iteration moves 88 instead of 120 bytes per unknown
+// and touches seven vectors instead of nine: 117 MB instead of 151 MB on the
+// 2048 x 1024 design (28 tiles per CTA), which the 126 MB L2 holds; there an
+// iteration takes 41 instead of 75 us (FP64).
+// ---------------------------------------------------------------------------
+template <typename T>
+struct PcgStreamCount {
+  static constexpr int value = sizeof(T) == 8 ? 30 : 55;
+};
+
+template <typename T, int R>
+struct PcgStream {
+  static constexpr int kPW = kTileJ + 2, kPN = (kTileI + 2) * kPW;
+  T p[R][kPN];
+  int ring[R][kHalo];  // element offset of each ring point, -1: no unknown there
+  int origin[R];
+};
+
+template <typename T, int R, class Group>
+__device__ __forceinline__ int pcg_stream(const DesignView& d, Group& g, double* smem, char* tbuf, double rz,
+                                          double beta) {
+  using Sm = PcgStream<T, R>;
+  constexpr int kU = 4;
+  Sm& S = *reinterpret_cast<Sm*>(tbuf);
+  const Inner<T>& w = inner<T>(d);
+  const int M = d.M, N = d.N, P = d.P;
+  const int tilesJ = (N - 1 + kTileJ - 1) / kTileJ;
+  const int nt = tilesJ * ((M - 1 + kTileI - 1) / kTileI);
+  const int th = threadIdx.x, ty = th / kTileJ, tx = th % kTileJ;
+  const int nk = (int)g.rank < nt ? (nt - 1 - (int)g.rank) / (int)g.nblk + 1 : 0;
+  const int lo = ty * P + tx, ip = (ty + 1) * Sm::kPW + tx + 1;
+  unsigned long long on = 0;  // bit k: the thread's point in tile k is a pressure unknown
+  for (int k = 0; k < nk; ++k) {
+    const int t = (int)g.rank + k * (int)g.nblk;
+    const int i0 = 1 + (t / tilesJ) * kTileI, j0 = 1 + (t % tilesJ) * kTileJ;
+    const bool mine = i0 + ty <= M - 1 && j0 + tx <= N - 2;
+    on |= mine ? 1ull << k : 0ull;
+    if (th == 0) S.origin[k] = i0 * P + j0;
+    S.p[k][ip] = mine ? w.pp0[i0 * P + j0 + lo] : (T)0;
+  }
+  for (int e = th; e < nk * kHalo; e += kThreads) {
+    const int k = e / kHalo, q = e - k * kHalo, t = (int)g.rank + k * (int)g.nblk;
+    int a, b;
+    const int at = ring_place(q, a, b);
+    const int i = 1 + (t / tilesJ) * kTileI + a, j = 1 + (t % tilesJ) * kTileJ + b;
+    const bool unknown = i >= 1 && i <= M - 1 && j >= 1 && j <= N - 2;
+    S.ring[k][q] = unknown ? i * P + j : -1;
+    S.p[k][at] = unknown ? w.pp0[i * P + j] : (T)0;
+  }
+  __syncthreads();
+  int it = 1;
+  for (; it < d.maxPIter; ++it) {
+    // p = z + beta p (pressure_solver.cpp:181)
+    auto pk = [&](T zq, T pq) -> T { return (T)((double)zq + beta * (double)pq); };
+    for (int k0 = 0; k0 < nk; k0 += kU) {
+      T z[kU];
+#pragma unroll
+      for (int u = 0; u < kU; ++u)
+        z[u] = ((on >> (k0 + u)) & 1ull) ? w.pz[S.origin[k0 + u] + lo] : (T)0;
+#pragma unroll
+      for (int u = 0; u < kU; ++u)
+        if (k0 + u < nk) S.p[k0 + u][ip] = pk(z[u], S.p[k0 + u][ip]);
+    }
+#pragma unroll 4
+    for (int e = th; e < nk * kHalo; e += kThreads) {
+      const int k = e / kHalo, q = e - k * kHalo, o = S.ring[k][q];
+      int a, b;
+      T* dst = &S.p[k][ring_place(q, a, b)];
+      if (o >= 0) *dst = pk(__ldcg(w.pz + o), *dst);
+    }
+    __syncthreads();
+    double s1[1] = {0.0};
+    for (int k0 = 0; k0 < nk; k0 += kU) {
+      T cE[kU], cW[kU], cN[kU], cS[kU], dg[kU];
+#pragma unroll
+      for (int u = 0; u < kU; ++u) {
+        const int o = ((on >> (k0 + u)) & 1ull) ? S.origin[k0 + u] + lo : P + 1;
+        cE[u] = w.cx[o];
+        cW[u] = w.cx[o - 1];
+        cN[u] = w.cy[o];
+        cS[u] = w.cy[o - P];
+        dg[u] = w.pdiag[o];
+      }
+#pragma unroll
+      for (int u = 0; u < kU; ++u) {
+        if (!((on >> (k0 + u)) & 1ull)) continue;
+        const int o = S.origin[k0 + u] + lo;
+        const T* q = &S.p[k0 + u][ip];
+        const double pc = (double)q[0];
+        double Ap = 0.0;
+        Ap += -(double)cS[u] * (double)q[-Sm::kPW];
+        Ap += -(double)cW[u] * (double)q[-1];
+        Ap += (double)dg[u] * pc;
+        Ap += -(double)cE[u] * (double)q[1];
+        Ap += -(double)cN[u] * (double)q[Sm::kPW];
+        const T apt = (T)Ap;
+        w.pAp[o] = apt;
+        s1[0] += pc * (double)apt;
+      }
+    }
+    if (!g.template sync_reduce<1, 0u>(s1, smem)) return -1;
+    const double pAp = s1[0];
+    if (fabs(pAp) < 1e-20) break;
+    const double alpha = div_uniform(rz, pAp);
+    double s2[2] = {0.0, 0.0};  // |r|^2, r.z
+    for (int k0 = 0; k0 < nk; k0 += kU) {
+      T x[kU], r[kU], ap[kU], dg[kU];
+#pragma unroll
+      for (int u = 0; u < kU; ++u) {
+        const int o = ((on >> (k0 + u)) & 1ull) ? S.origin[k0 + u] + lo : P + 1;
+        x[u] = w.px[o];
+        r[u] = w.pr[o];
+        ap[u] = w.pAp[o];
+        dg[u] = w.pdiag[o];
+      }
+#pragma unroll
+      for (int u = 0; u < kU; ++u) {
+        if (!((on >> (k0 + u)) & 1ull)) continue;
+        const int o = S.origin[k0 + u] + lo;
+        w.px[o] = (T)((double)x[u] + alpha * (double)S.p[k0 + u][ip]);
+        const T rt = residual_of(r[u], alpha, ap[u]);
+        w.pr[o] = rt;
+        const double rr = (double)rt;
+        s2[0] += rr * rr;
+        const T z = precond_of(rt, dg[u]);
+        w.pz[o] = z;
+        s2[1] += rr * (double)z;
+      }
+    }
+    if (!g.template sync_reduce<2, 0u>(s2, smem)) return -1;
+    if (s2[0] < d.pStop) break;
+    beta = div_uniform(s2[1], rz);
+    rz = s2[1];
+  }
+  return it;
+}
+
+inline __host__ __device__ int pcg_tiles_of(int M, int N) {
+  return ((M - 1 + kTileI - 1) / kTileI) * ((N - 1 + kTileJ - 1) / kTileJ);
+}
+// The PCG form of an M x N design on nblk CTAs.
+template <typename T>
+inline __host__ __device__ int pcg_form(int M, int N, int nblk) {
+  const int tiles = pcg_tiles_of(M, N);
+  return tiles <= kFewTiles * nblk ? kFew : tiles <= PcgTileCount<T>::value * nblk ? kMany : kLarge;
+}
+
+// ---------------------------------------------------------------------------
+// PCG as the reference runs it (pressure_solver.cpp:121-184): two grid-wide
+// reductions per iteration (p.Ap, then |r|^2 and r.z).  Phase P1 forms
+// p = z + beta p on the fly for the 5-point stencil and Ap; phase P2 updates
+// x, r, z.  rz0 = r0.z0 and pAp0 = p0.A p0 come from phase C.  From iteration
+// 1 on the CTAs hold their tiles on chip (pcg_tiles), or p of them (pcg_stream),
+// when they fit, else read global memory (pcg_global).  Returns the reference's iteration count, or -1
+// if a wait failed.
+// ---------------------------------------------------------------------------
+template <typename T, int Carry, class Group>
+__device__ __forceinline__ int pcg_two_reductions(const DesignView& d, Group& g, double* smem, char* tbuf, double rz0,
+                                                  double pAp0) {
+  constexpr int kTiles = PcgTileCount<T>::value, kStream = PcgStreamCount<T>::value;
+  if (d.maxPIter == 0 || fabs(pAp0) < 1e-20) return no_update<T>(d, g);
+  const int form = pcg_form<T>(d.M, d.N, (int)g.nblk);
+  const double alpha = div_uniform(rz0, pAp0);
+  double s2[2] = {0.0, 0.0};
+  bool ok;
+  if constexpr ((Carry & kLarge) == 0) ok = pcg_first<T, false>(d, g, smem, alpha, s2);
+  else if constexpr ((Carry & kForms) == kLarge) ok = pcg_first<T, true>(d, g, smem, alpha, s2);
+  else ok = form == kLarge ? pcg_first<T, true>(d, g, smem, alpha, s2) : pcg_first<T, false>(d, g, smem, alpha, s2);
+  if (!ok) return -1;
+  if (s2[0] < d.pStop) return 0;
+  if (d.maxPIter == 1) return 1;
+  const double rz = s2[1], beta = div_uniform(rz, rz0);
+  if constexpr ((Carry & kFew) != 0)
+    if ((Carry & kForms) == kFew || form == kFew) return pcg_tiles<T, kFewTiles>(d, g, smem, tbuf, alpha, rz, beta);
+  if constexpr ((Carry & kMany) != 0)
+    if ((Carry & kForms) == kMany || form == kMany) return pcg_tiles<T, kTiles>(d, g, smem, tbuf, alpha, rz, beta);
+  if constexpr ((Carry & kLarge) != 0)
+    return pcg_tiles_of(d.M, d.N) <= kStream * (int)g.nblk ? pcg_stream<T, kStream>(d, g, smem, tbuf, rz, beta)
+                                                          : pcg_global<T>(d, g, smem, rz, beta);
+  return -1;
 }
 
 // ---------------------------------------------------------------------------
@@ -1931,7 +2030,7 @@ __device__ __forceinline__ double final_velocity(double vel, T xf) {
 
 // Returns false when a wait failed.  rc: residU, residV, residMass,
 // residMassDof, non-finite flag (max); r.z, p.Ap (sum).
-template <typename T, class Group>
+template <typename T, bool Opt, class Group>
 __device__ bool mass_phase(const DesignView& d, Group& g, double* smem, char* tbuf, const T* xfU, const T* xfV,
                            int mapXU, int mapXV, double (&rc)[7]) {
   const Inner<T>& w = inner<T>(d);
@@ -2053,13 +2152,12 @@ __device__ bool mass_phase(const DesignView& d, Group& g, double* smem, char* tb
           w.cy[o] = (T)aN;
           const T rt = (T)b;
           w.pr[o] = rt;
-          w.px[o] = (T)0.0;
           const double rr = (double)rt;
           const T z = (T)z0(i, j);  // formed from the same stored values above
-          if (d.pcgSingleReduction) {
+          if (Opt && d.pcgSingleReduction) {
             w.cU[o + d.planeStride] = z;  // u0 = M^-1 r0 of the single-reduction recurrences
+            w.px[o] = (T)0.0;
           } else {
-            w.pz[o] = z;
             w.pp0[o] = z;
           }
           rc[5] += rr * (double)z;
@@ -2269,7 +2367,9 @@ constexpr size_t tile_smem_bytes() {
   constexpr size_t m0 = a > c ? a : c;
   constexpr size_t m = m0 > bb ? m0 : bb;
   constexpr size_t t = m > dd ? m : dd;
-  constexpr size_t q = CPS_SMEM_PCG ? sizeof(PcgSmem<T, SmemTiles<T>::value>) : 0;  // the PCG reuses the buffers
+  // the PCG reuses the buffers
+  constexpr size_t q0 = sizeof(PcgTiles<T, PcgTileCount<T>::value>), q1 = sizeof(PcgStream<T, PcgStreamCount<T>::value>);
+  constexpr size_t q = q0 > q1 ? q0 : q1;
   return t > q ? t : q;
 }
 
@@ -2297,7 +2397,7 @@ __device__ __forceinline__ bool tile_buffer_aligned(const char* dyn, int* status
 // pressure-drop gate, or a non-finite residual), -1 when the group must stop
 // because a device-side wait failed.
 // ---------------------------------------------------------------------------
-template <typename T, class Group, bool Monitor = false, bool Pseudo = true>
+template <typename T, class Group, bool Monitor = false, bool Pseudo = true, int Carry = kAll>
 __device__ int outer_iteration(const DesignView& d, Group& g, double* smem, char* tbuf, double* out,
                                bool lastIter, bool stopOnConv, double eps, int iter = 0, double* dplog = nullptr,
                                int* dpConverged = nullptr, PseudoRun* pr = nullptr, SweepHint* hint = nullptr) {
@@ -2305,7 +2405,8 @@ __device__ int outer_iteration(const DesignView& d, Group& g, double* smem, char
   const int M = d.M, N = d.N, P = d.P;
   // ---- A: assembly + sweep 1 (or the explicit update) ----
   const double cfl = (Pseudo && d.pseudo && pr) ? pr->cfl : 0.0;
-  const bool expl = d.momExplicit != 0;
+  constexpr bool opt = (Carry & kOptions) != 0;
+  const bool expl = opt && d.momExplicit != 0;
   const bool anySweep = !expl && d.maxMomIter > 0;
   // Rows are stored in phase A when the last outer iteration needed a second
   // sweep of that component (the sweep counts change slowly); otherwise a
@@ -2367,7 +2468,7 @@ __device__ int outer_iteration(const DesignView& d, Group& g, double* smem, char
               s[1] += storeV ? sweep_point<false, T>(d, i, j, xinV, xoutV)
                              : sweep2_point<false, T, Pseudo>(d, L, i, j, cfl, xinV, xoutV, store);
           });
-    } else if (d.tm && d.stageSweeps) {
+    } else if (opt && d.tm && d.stageSweeps) {
       using LB = LayoutB<T>;
       const long long ps = d.planeStride;
       const int mapXU = (k & 1) ? kTmXU0_B : kTmXU1_B, mapXV = (k & 1) ? kTmXV0_B : kTmXV1_B;
@@ -2422,7 +2523,7 @@ __device__ int outer_iteration(const DesignView& d, Group& g, double* smem, char
   const T* xfV = (kV & 1) ? w.xV1 : w.xV0;
   // ---- C: scatter, BCs, mass residual, PCG set-up ----
   double rc[7] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-  if (!mass_phase<T>(d, g, smem, tbuf, xfU, xfV, (kU & 1) ? kTmXU1_C : kTmXU0_C, (kV & 1) ? kTmXV1_C : kTmXV0_C, rc))
+  if (!mass_phase<T, opt>(d, g, smem, tbuf, xfU, xfV, (kU & 1) ? kTmXU1_C : kTmXU0_C, (kV & 1) ? kTmXV1_C : kTmXV0_C, rc))
     return -1;
   // std::max({residU, residV, residMass}) (iterations.cpp:525); the stop test
   // uses the mass imbalance over the pressure unknowns.
@@ -2457,25 +2558,14 @@ __device__ int outer_iteration(const DesignView& d, Group& g, double* smem, char
     }
   }
   // ---- P: Jacobi-preconditioned CG ----
-  if (d.pcgSingleReduction) {
+  if (opt && d.pcgSingleReduction) {
     const int its = pcg_single_reduction<T>(d, g, smem, rc[5], rc[6]);
     if (its < 0) return -1;
     if (threadIdx.x == 0) out[5] = its;
   } else {
-    const int tiles = ((M - 1 + kTileI - 1) / kTileI) * ((N - 1 + kTileJ - 1) / kTileJ);
-    constexpr int kS = SmemTiles<T>::value;
-    int its;
-    if (tiles <= kResidentTiles * (int)g.nblk)
-      its = pcg_resident<T, kResidentTiles>(d, g, smem, rc[5], rc[6]);
-    else if (CPS_SMEM_PCG && tiles <= kS * (int)g.nblk && (!hint || hint->kP >= 2))
-      // the shared-memory form pays when the PCG runs several iterations (its
-      // loading costs about one); the last outer iteration's count decides
-      its = pcg_smem<T, kS>(d, g, smem, tbuf, rc[5], rc[6]);
-    else
-      its = pcg_two_reductions<T>(d, g, smem, rc[5], rc[6]);
+    const int its = pcg_two_reductions<T, Carry>(d, g, smem, tbuf, rc[5], rc[6]);
     if (its < 0) return -1;
     if (threadIdx.x == 0) out[5] = its;
-    if (hint) hint->kP = its;
   }
   // ---- D: pressure and velocity correction ----
   if (!correct_fields<T>(d, g, tbuf)) return -1;

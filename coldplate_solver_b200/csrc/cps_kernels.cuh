@@ -1,6 +1,6 @@
 // The persistent kernels.  Their instantiations are compiled in translation
-// units of their own (cps_grid_f64.cu, cps_grid_f32.cu, cps_batch_f64.cu,
-// cps_batch_f32.cu), side by side: together in one they take minutes.
+// units of their own (cps_grid_*.cu, cps_batch_*.cu), side by side: together in
+// one they take minutes.
 #pragma once
 #include "cps_device.cuh"
 
@@ -8,7 +8,8 @@
 // separate instantiation: compiling it into the plain kernel slowed every
 // outer iteration by 60 % on B200).  Pseudo: the pseudo-transient term and the
 // CFL controllers compiled in (their registers spill the plain kernel's).
-template <typename T, bool Monitor, bool Pseudo>
+// Carry: the PCG forms and options compiled in (cps::Carries).
+template <typename T, bool Monitor, bool Pseudo, int Carry>
 __global__ void __launch_bounds__(cps::kThreads, CPS_MIN_BLOCKS) cps_grid_kernel(cps::DesignView d, cps::RunControl rc,
                                                                 cps::GridBarrier* bar, double* red) {
   __shared__ double smem[(Monitor ? cps::kPlaneSums : cps::kRedWidth) * 8];
@@ -20,9 +21,9 @@ __global__ void __launch_bounds__(cps::kThreads, CPS_MIN_BLOCKS) cps_grid_kernel
   cps::tma_barriers_init();
   cps::load_pseudo(d, s_pr);
   __syncthreads();
-  cps::SweepHint hint{2, 2, 2};
+  cps::SweepHint hint{2, 2};
   for (int it = 0; it < rc.n_outer; ++it) {
-    const int r = cps::outer_iteration<T, cps::GridGroup, Monitor, Pseudo>(
+    const int r = cps::outer_iteration<T, cps::GridGroup, Monitor, Pseudo, Carry>(
         d, g, smem, tile_smem, out, it + 1 == rc.n_outer, rc.stop_on_conv != 0, rc.eps, rc.iter0 + it,
         rc.dplog ? rc.dplog + (size_t)4 * it : nullptr, rc.dp_converged, &s_pr, &hint);
     if (r < 0) return;
@@ -36,7 +37,7 @@ __global__ void __launch_bounds__(cps::kThreads, CPS_MIN_BLOCKS) cps_grid_kernel
 
 // Batched solves: each cluster takes the next design from the queue and runs
 // its outer iterations to convergence or to the item's budget.
-template <typename T, bool Pseudo>
+template <typename T, bool Options>
 __global__ void __launch_bounds__(cps::kThreads) cps_cluster_kernel(const cps::BatchItem* __restrict__ items,
                                                                    const int* __restrict__ order, int n_items,
                                                                    int* queue, cps::BatchResult* results) {
@@ -70,9 +71,9 @@ __global__ void __launch_bounds__(cps::kThreads) cps_cluster_kernel(const cps::B
     g.status = &res->status;
     if (threadIdx.x < 8) out[threadIdx.x] = 0.0;
     int done = 0;
-    cps::SweepHint hint{2, 2, 2};
+    cps::SweepHint hint{2, 2};
     for (int it = 0; it < item.n_outer; ++it) {
-      const int r = cps::outer_iteration<T, cps::ClusterGroup, false, Pseudo>(
+      const int r = cps::outer_iteration<T, cps::ClusterGroup, false, Options, Options ? cps::kAll : cps::kForms>(
           item.view, g, smem, tile_smem, out, it + 1 == item.n_outer, item.stop_on_conv != 0, item.eps, item.iter0 + it,
           nullptr, nullptr, &s_pr, &hint);
       done = it + 1;
@@ -96,7 +97,7 @@ __global__ void __launch_bounds__(cps::kThreads) cps_cluster_kernel(const cps::B
 // time and runs each with the bounded software barrier of its own counter.
 // The group count sets how many designs are in flight (and so the in-flight
 // working set against the 126 MB L2); K sets how many CTAs share one design.
-template <typename T, bool Pseudo>
+template <typename T, bool Options>
 __global__ void __launch_bounds__(cps::kThreads, CPS_MIN_BLOCKS) cps_group_kernel(const cps::BatchItem* __restrict__ items,
                                                                     const int* __restrict__ order, int n_items,
                                                                     int* queue, cps::BatchResult* results,
@@ -134,9 +135,9 @@ __global__ void __launch_bounds__(cps::kThreads, CPS_MIN_BLOCKS) cps_group_kerne
     g.status = &res->status;
     if (threadIdx.x < 8) out[threadIdx.x] = 0.0;
     int done = 0;
-    cps::SweepHint hint{2, 2, 2};
+    cps::SweepHint hint{2, 2};
     for (int it = 0; it < item.n_outer; ++it) {
-      const int r = cps::outer_iteration<T, cps::GridGroup, false, Pseudo>(
+      const int r = cps::outer_iteration<T, cps::GridGroup, false, Options, Options ? cps::kAll : cps::kForms>(
           item.view, g, smem, tile_smem, out, it + 1 == item.n_outer, item.stop_on_conv != 0, item.eps, item.iter0 + it,
           nullptr, nullptr, &s_pr, &hint);
       if (r < 0) return;  // a bounded wait expired; the design's status says so
@@ -159,7 +160,7 @@ __global__ void __launch_bounds__(cps::kThreads, CPS_MIN_BLOCKS) cps_group_kerne
 // designs.  CTAs [first[g], first[g+1]) form group g and run design which[g]
 // to convergence or to its budget with the bounded software barrier of their
 // own counter; their reduction ring starts at first[g] ring rows.
-template <typename T, bool Pseudo>
+template <typename T, bool Options>
 __global__ void __launch_bounds__(cps::kThreads, CPS_MIN_BLOCKS) cps_wave_kernel(const cps::BatchItem* __restrict__ items,
                                                                    const int* __restrict__ first,
                                                                    const int* __restrict__ which, int groups,
@@ -192,9 +193,9 @@ __global__ void __launch_bounds__(cps::kThreads, CPS_MIN_BLOCKS) cps_wave_kernel
                    blockIdx.x - (unsigned)first[grp], (unsigned)K, 0u, 0ull};
   if (threadIdx.x < 8) out[threadIdx.x] = 0.0;
   int done = 0;
-  cps::SweepHint hint{2, 2, 2};
+  cps::SweepHint hint{2, 2};
   for (int it = 0; it < item.n_outer; ++it) {
-    const int r = cps::outer_iteration<T, cps::GridGroup, false, Pseudo>(
+    const int r = cps::outer_iteration<T, cps::GridGroup, false, Options, Options ? cps::kAll : cps::kForms>(
         item.view, g, smem, tile_smem, out, it + 1 == item.n_outer, item.stop_on_conv != 0, item.eps, item.iter0 + it,
         nullptr, nullptr, &s_pr, &hint);
     if (r < 0) return;  // a bounded wait expired; the design's status says so
@@ -211,19 +212,26 @@ __global__ void __launch_bounds__(cps::kThreads, CPS_MIN_BLOCKS) cps_wave_kernel
   }
 }
 
-// Every instantiation the library launches, storage type T.
+// Every instantiation the library launches, storage type T.  Batches carry all
+// PCG forms (their designs differ in size); Options adds the pseudo-transient
+// term, the CFL controllers and the options of cps::kOptions.
+#define CPS_GRID_KERNEL(PRE, T, MONITOR, PSEUDO, CARRY)                                                             \
+  PRE template __global__ void cps_grid_kernel<T, MONITOR, PSEUDO, CARRY>(cps::DesignView, cps::RunControl,         \
+                                                                          cps::GridBarrier*, double*);
 #define CPS_GRID_KERNELS(PRE, T)                                                                                    \
-  PRE template __global__ void cps_grid_kernel<T, false, false>(cps::DesignView, cps::RunControl, cps::GridBarrier*, \
-                                                                double*);                                           \
-  PRE template __global__ void cps_grid_kernel<T, false, true>(cps::DesignView, cps::RunControl, cps::GridBarrier*,  \
-                                                               double*);                                            \
-  PRE template __global__ void cps_grid_kernel<T, true, true>(cps::DesignView, cps::RunControl, cps::GridBarrier*,   \
-                                                              double*);
-#define CPS_BATCH_KERNELS_OF(PRE, T, PSEUDO)                                                                        \
-  PRE template __global__ void cps_cluster_kernel<T, PSEUDO>(const cps::BatchItem*, const int*, int, int*,           \
-                                                             cps::BatchResult*);                                    \
-  PRE template __global__ void cps_group_kernel<T, PSEUDO>(const cps::BatchItem*, const int*, int, int*,             \
-                                                           cps::BatchResult*, cps::GridBarrier*, double*, int*, int); \
-  PRE template __global__ void cps_wave_kernel<T, PSEUDO>(const cps::BatchItem*, const int*, const int*, int,         \
-                                                          cps::BatchResult*, cps::GridBarrier*, double*);
-#define CPS_BATCH_KERNELS(PRE, T) CPS_BATCH_KERNELS_OF(PRE, T, false) CPS_BATCH_KERNELS_OF(PRE, T, true)
+  CPS_GRID_KERNEL(PRE, T, false, false, cps::kFew)                                                                  \
+  CPS_GRID_KERNEL(PRE, T, false, false, cps::kMany)                                                                 \
+  CPS_GRID_KERNEL(PRE, T, false, false, cps::kLarge)
+#define CPS_GRID_OPTION_KERNELS(PRE, T)                                                                             \
+  CPS_GRID_KERNEL(PRE, T, false, true, cps::kAll)                                                                   \
+  CPS_GRID_KERNEL(PRE, T, true, true, cps::kAll)
+#define CPS_BATCH_KERNELS_OF(PRE, T, OPTIONS)                                                                       \
+  PRE template __global__ void cps_cluster_kernel<T, OPTIONS>(const cps::BatchItem*, const int*, int, int*,          \
+                                                              cps::BatchResult*);                                   \
+  PRE template __global__ void cps_group_kernel<T, OPTIONS>(const cps::BatchItem*, const int*, int, int*,            \
+                                                            cps::BatchResult*, cps::GridBarrier*, double*, int*,    \
+                                                            int);                                                   \
+  PRE template __global__ void cps_wave_kernel<T, OPTIONS>(const cps::BatchItem*, const int*, const int*, int,        \
+                                                           cps::BatchResult*, cps::GridBarrier*, double*);
+#define CPS_BATCH_KERNELS(PRE, T) CPS_BATCH_KERNELS_OF(PRE, T, false)
+#define CPS_BATCH_OPTION_KERNELS(PRE, T) CPS_BATCH_KERNELS_OF(PRE, T, true)
