@@ -386,11 +386,7 @@ class Solver:
         nd = ctypes.c_int(0)
         uin = self.inletVelocity if inletVelocity is None else inletVelocity
         self._check(self.lib.cps_solve(self.ctx, uin, max_outer, eps, hist, ctypes.byref(nd)))
-        out = np.zeros((nd.value, 8))
-        for k in range(nd.value):
-            h = hist[k]
-            out[k] = (h.residU, h.residV, h.residMass, h.residMassDof, h.err, h.pIters, h.uSweeps, h.vSweeps)
-        return out
+        return history_to_array(hist, nd.value)
 
     def set_pseudo(self, design: Optional[Design] = None) -> None:
         """cps_set_pseudo with the pseudo-transient settings of ``design``
@@ -439,11 +435,7 @@ class Solver:
         uin = self.inletVelocity if inletVelocity is None else inletVelocity
         self._check(self.lib.cps_solve_monitored(self.ctx, uin, max_outer, eps, hist, _dptr(dp), ctypes.byref(nd),
                                                  ctypes.byref(conv)))
-        out = np.zeros((nd.value, 8))
-        for k in range(nd.value):
-            h = hist[k]
-            out[k] = (h.residU, h.residV, h.residMass, h.residMassDof, h.err, h.pIters, h.uSweeps, h.vSweeps)
-        return out, dp[: nd.value].copy(), bool(conv.value)
+        return history_to_array(hist, nd.value), dp[: nd.value].copy(), bool(conv.value)
 
     def sample_plane(self, x: float) -> np.ndarray:
         pl = CpsPlane()
@@ -458,18 +450,23 @@ class Solver:
 
     def download(self) -> Dict[str, np.ndarray]:
         shapes = field_shapes(self.design.M, self.design.N)
-        out = {k: np.zeros(s) for k, s in shapes.items()}
+        out = {k: np.empty(s) for k, s in shapes.items()}
         self._check(self.lib.cps_download_fields(self.ctx, *[_dptr(out[k]) for k in
                                                             ("u", "v", "p", "pStar", "uStar", "vStar", "dE", "dN")],
                                                  CPS_ROW_MAJOR))
         return out
 
 
+_STEP_DTYPE = np.dtype(CpsStepOut)
+
+
 def history_to_array(hist, n: int) -> np.ndarray:
-    out = np.zeros((n, 8))
-    for k in range(n):
-        h = hist[k]
-        out[k] = (h.residU, h.residV, h.residMass, h.residMassDof, h.err, h.pIters, h.uSweeps, h.vSweeps)
+    """The first n steps of a CpsStepOut array as rows: residU, residV,
+    residMass, residMassDof, err, pIters, uSweeps, vSweeps."""
+    a = np.frombuffer(hist, dtype=_STEP_DTYPE, count=n) if n > 0 else np.zeros(0, dtype=_STEP_DTYPE)
+    out = np.empty((n, 8))
+    for j, (name, _) in enumerate(CpsStepOut._fields_):
+        out[:, j] = a[name]
     return out
 
 
