@@ -79,6 +79,7 @@ struct cps_ctx {
   int ramp_steps = 0;        // inlet velocity ramp of cps_solve (0: off)
   int iter = 0;              // outer-loop iteration index of the next iteration (monitor and gate)
   int grid = 0;
+  bool cluster = false;      // the PCG may run on one thread-block cluster (cps::kCluster)
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   double kernel_ms = 0.0;
   long long launches = 0, outer_done = 0;
@@ -380,20 +381,34 @@ void set_step_inputs(cps_ctx* c, double Uin) {
   c->view.maxVel = 3.0 * std::max(std::fabs(Uin), 0.1);  // iterations.cpp:104
 }
 
-// The single-design kernels of a storage type: one per PCG form on the default
-// path, then the ones that carry every option, without and with the monitor.
-template <typename T>
-const void* grid_kernel(int k) {
-  switch (k) {
-    case 0: return (const void*)cps_grid_kernel<T, false, false, cps::kFew>;
-    case 1: return (const void*)cps_grid_kernel<T, false, false, cps::kMany>;
-    case 2: return (const void*)cps_grid_kernel<T, false, false, cps::kLarge>;
-    case 3: return (const void*)cps_grid_kernel<T, false, true, cps::kAll>;
-    default: return (const void*)cps_grid_kernel<T, true, true, cps::kAll>;
-  }
+// The single-design kernels of a storage type, each with the dynamic shared
+// memory it needs: one per PCG form on the default path, then the ones that
+// carry every option, without and with the monitor, then the one whose PCG
+// runs on one cluster (8 x 32 tiles only).
+struct GridKernel {
+  const void* fn;
+  size_t smem;
+};
+template <typename T, bool Monitor, bool Pseudo, int Carry>
+GridKernel grid_kernel() {
+  return {(const void*)cps_grid_kernel<T, Monitor, Pseudo, Carry>, cps::kernel_smem_bytes<T, Carry, Monitor>()};
 }
-constexpr int kGridKernels = 5;
-const void* grid_kernel_of(int precision, int k) {
+enum GridKernels : int { kGridFew, kGridMany, kGridLarge, kGridOptions, kGridMonitor, kGridKernels, kGridCluster = kGridKernels };
+template <typename T>
+GridKernel grid_kernel(int k) {
+  switch (k) {
+    case kGridFew: return grid_kernel<T, false, false, cps::kFew>();
+    case kGridMany: return grid_kernel<T, false, false, cps::kMany>();
+    case kGridLarge: return grid_kernel<T, false, false, cps::kLarge>();
+    case kGridOptions: return grid_kernel<T, false, true, cps::kAll>();
+    case kGridMonitor: return grid_kernel<T, true, true, cps::kAll>();
+#if CPS_TILE_J == 32
+    case kGridCluster: return grid_kernel<T, false, false, cps::kCluster>();
+#endif
+  }
+  return {nullptr, 0};
+}
+GridKernel grid_kernel_of(int precision, int k) {
   return precision == CPS_MIXED ? grid_kernel<float>(k) : grid_kernel<double>(k);
 }
 
@@ -402,12 +417,13 @@ bool has_options(const cps::DesignView& v) {
   return v.pseudo != 0 || v.momExplicit != 0 || v.pcgSingleReduction != 0 || v.stageSweeps != 0;
 }
 
-const void* grid_kernel_for(const cps_ctx* c) {
-  if (c->view.dpMonitor) return grid_kernel_of(c->precision, 4);
-  if (has_options(c->view)) return grid_kernel_of(c->precision, 3);
+int grid_kernel_for(const cps_ctx* c) {
+  if (c->view.dpMonitor) return kGridMonitor;
+  if (has_options(c->view)) return kGridOptions;
+  if (c->cluster) return kGridCluster;
   const int form = c->precision == CPS_MIXED ? cps::pcg_form<float>(c->M, c->N, c->grid)
                                              : cps::pcg_form<double>(c->M, c->N, c->grid);
-  return grid_kernel_of(c->precision, form == cps::kFew ? 0 : form == cps::kMany ? 1 : 2);
+  return form == cps::kFew ? kGridFew : form == cps::kMany ? kGridMany : kGridLarge;
 }
 
 // Dynamic shared memory of the persistent kernels (tile staging buffers).
@@ -423,6 +439,58 @@ bool allow_smem(cps_ctx* c, const void* fn, size_t bytes) {
 void to_step_out(const double* h, cps_step_out* o) {
   o->residU = h[0]; o->residV = h[1]; o->residMass = h[2]; o->residMassDof = h[3]; o->err = h[4];
   o->pIters = (int)h[5]; o->uSweeps = (int)h[6]; o->vSweeps = (int)h[7];
+}
+
+// The persistent kernel's launch: cooperative (all CTAs co-resident), in
+// clusters where its PCG runs on one.
+cudaError_t launch_grid(const cps_ctx* c, void** args) {
+  const int k = grid_kernel_for(c);
+  const GridKernel kern = grid_kernel_of(c->precision, k);
+  const bool cluster = k == kGridCluster;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[2];
+  cfg.gridDim = dim3(cluster ? (unsigned)round_up(c->grid, cps::kClusterCtas) : (unsigned)c->grid);
+  cfg.blockDim = dim3(cps::kThreads);
+  cfg.dynamicSmemBytes = kern.smem;
+  cfg.stream = c->stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster ? 2 : 1;
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cps::kClusterCtas;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  return cudaLaunchKernelExC(&cfg, kern.fn, args);
+}
+
+// Whether a design's PCG runs on one cluster: one tile per CTA, tiles enough
+// for the cluster's CTAs and no more than its warps, a cap that leaves it
+// iterations to run (the form costs one more grid barrier) and that it meets
+// well inside the grid barrier's time limit, and room for the launch's
+// clusters at one CTA per SM (seven of 16 CTAs on B200).
+bool use_cluster(const cps_ctx* c, const cps_desc* d) {
+  const GridKernel kern = grid_kernel_of(c->precision, kGridCluster);
+  const int tiles = cps::pcg_tiles_of(c->M, c->N);
+  if (!kern.fn || c->grid != tiles || tiles < cps::kClusterCtas || tiles > cps::kClusterTiles || d->maxPressureIter < 3 ||
+      d->maxPressureIter > 100000)
+    return false;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  cfg.gridDim = dim3((unsigned)round_up(tiles, cps::kClusterCtas));
+  cfg.blockDim = dim3(cps::kThreads);
+  cfg.dynamicSmemBytes = kern.smem;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = cps::kClusterCtas;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  int clusters = 0;
+  const bool ok = cudaFuncSetAttribute(kern.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kern.smem) == cudaSuccess &&
+                  cudaFuncSetAttribute(kern.fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                  cudaOccupancyMaxActiveClusters(&clusters, kern.fn, &cfg) == cudaSuccess &&
+                  clusters * cps::kClusterCtas >= (int)cfg.gridDim.x;
+  if (!ok) cudaGetLastError();  // the other forms need none of it
+  return ok;
 }
 
 cps_status run(cps_ctx* c, int n_outer, int stop_on_conv, double eps, cps_step_out* hist, int* n_done,
@@ -443,15 +511,13 @@ cps_status run(cps_ctx* c, int n_outer, int stop_on_conv, double eps, cps_step_o
       }
     }
     cps::RunControl rc{chunk, stop_on_conv, eps, c->dhist, c->dndone, c->dstatus, c->iter,
-                       monitor ? c->dplog : nullptr, c->dstatus + 2};
+                       monitor ? c->dplog : nullptr, c->dstatus + 2, c->grid};
     if (!cuda_ok(c, cudaMemsetAsync(c->dndone, 0, 2 * sizeof(int), c->stream), "memset") ||
         !cuda_ok(c, cudaMemsetAsync(c->bar, 0, sizeof(cps::GridBarrier), c->stream), "memset"))
       return CPS_ERR_CUDA;
     void* args[] = {&c->view, &rc, &c->bar, &c->red};
     if (!cuda_ok(c, cudaEventRecord(c->ev0, c->stream), "event")) return CPS_ERR_CUDA;
-    if (!cuda_ok(c, cudaLaunchCooperativeKernel(grid_kernel_for(c), dim3(c->grid), dim3(cps::kThreads),
-                                                args, tile_smem_for(c->precision), c->stream), "cooperative launch"))
-      return CPS_ERR_CUDA;
+    if (!cuda_ok(c, launch_grid(c, args), "cooperative launch")) return CPS_ERR_CUDA;
     if (!cuda_ok(c, cudaEventRecord(c->ev1, c->stream), "event")) return CPS_ERR_CUDA;
     if (!cuda_ok(c, cudaMemcpyAsync(c->hflags, c->dstatus, 3 * sizeof(int), cudaMemcpyDeviceToHost, c->stream), "d2h"))
       return CPS_ERR_CUDA;
@@ -711,11 +777,10 @@ cps_status cps_create(const cps_desc* d, cps_ctx** out) {
   int per_sm = 0, sms = 0;
   for (int k = 0; k < kGridKernels; ++k) {
     // the kernels are interchangeable within a design, so the grid is what all of them allow
-    const void* fn = grid_kernel_of(d->precision, k);
+    const GridKernel kern = grid_kernel_of(d->precision, k);
     int n = 0;
-    if (!allow_smem(c, fn, tile_smem_for(d->precision)) ||
-        !cuda_ok(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, cps::kThreads, tile_smem_for(d->precision)),
-                 "occupancy"))
+    if (!allow_smem(c, kern.fn, kern.smem) ||
+        !cuda_ok(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern.fn, cps::kThreads, kern.smem), "occupancy"))
       return bail(CPS_ERR_CUDA);
     per_sm = k == 0 ? n : std::min(per_sm, n);
   }
@@ -731,6 +796,7 @@ cps_status cps_create(const cps_desc* d, cps_ctx** out) {
   grid = std::min(grid, cap);
   grid = std::max(1, std::min(grid, tiles));
   c->grid = grid;
+  c->cluster = use_cluster(c, d);
   *out = c;
   return CPS_OK;
 }
@@ -946,9 +1012,9 @@ cps_status cps_set_dp_monitor(cps_ctx* c, const cps_dp_monitor* m) {
   if (m->window < 1 || m->slope_window < 0 || m->ramp_steps < 0 || !(m->percent >= 0.0))
     return fail(c, CPS_ERR_ARG, "dp monitor: window >= 1, slope_window >= 0, ramp_steps >= 0, percent >= 0");
   const size_t slots = (size_t)m->window + (size_t)(m->slope_gate ? m->slope_window : 0);
-  if (slots * sizeof(double) > tile_smem_for(c->precision))
-    return fail(c, CPS_ERR_ARG, "dp monitor: window + slope_window exceeds " +
-                                    std::to_string(tile_smem_for(c->precision) / sizeof(double)) + " values");
+  const size_t most = c->precision == CPS_MIXED ? cps::window_values<float>() : cps::window_values<double>();
+  if (slots > most)
+    return fail(c, CPS_ERR_ARG, "dp monitor: window + slope_window exceeds " + std::to_string(most) + " values");
   if (c->ddphist) cudaFree(c->ddphist);
   c->ddphist = nullptr;
   if (!cuda_ok(c, cudaMalloc(&c->ddphist, std::max<size_t>(slots, 1) * sizeof(double)), "cudaMalloc")) return CPS_ERR_OOM;

@@ -113,7 +113,7 @@ enum TmaMap : int {
 // from every phase (all forms and options in one kernel: 165 bytes of spills,
 // late outer iterations 5 % slower), so the host launches the least that a
 // design needs.
-enum Carries : int { kFew = 1, kMany = 2, kLarge = 4, kForms = 7, kOptions = 8, kAll = 15 };
+enum Carries : int { kFew = 1, kMany = 2, kLarge = 4, kForms = 7, kOptions = 8, kAll = 15, kCluster = 16 };
 
 enum DeviceStatus : int { kStatusOk = 0, kStatusTimeout = 1, kStatusDiverged = 2 };
 
@@ -210,6 +210,7 @@ struct RunControl {
   int iter0;          // the outer loop's iteration index of this launch's first iteration
   double* dplog;      // n_outer x 4 (core total, full total, core static, full static dP) or null
   int* dp_converged;  // set when the pressure-drop gate stopped the loop
+  int ctas;           // CTAs that run the design (a cluster launch may have a few more)
 };
 
 // One entry of the batched (cluster) kernel's work list.
@@ -271,6 +272,13 @@ __device__ __forceinline__ double clampd(double v, double lo, double hi) { retur
 // quotients below 2^-960 the remainder may underflow and the last bit is not
 // guaranteed; an infinite numerator or an overflowing quotient gives q.
 // ---------------------------------------------------------------------------
+// c ? a : b with both evaluated: no branch for the compiler to put around a
+// division, so that a thread's divisions overlap.
+__device__ __forceinline__ double select(bool c, double a, double b) {
+  double r;
+  asm("{\n .reg .pred p;\n setp.ne.s32 p, %3, 0;\n selp.f64 %0, %1, %2, p;\n}" : "=d"(r) : "d"(a), "d"(b), "r"((int)c));
+  return r;
+}
 // One Newton step of y towards 1/b.
 __device__ __forceinline__ double recip_step(double b, double y) { return __fma_rn(y, __fma_rn(-b, y, 1.0), y); }
 __device__ __forceinline__ double recip(double b) {
@@ -282,7 +290,7 @@ __device__ __forceinline__ double recip(double b) {
 __device__ __forceinline__ double div_rn(double a, double b, double y) {
   const double q = a * y;
   const double v = __fma_rn(__fma_rn(-b, q, a), y, q);
-  return (__double2hiint(v) & 0x7ff00000) == 0x7ff00000 ? q : v;
+  return select((__double2hiint(v) & 0x7ff00000) == 0x7ff00000, q, v);
 }
 __device__ __forceinline__ double div_rn(double a, double b) { return div_rn(a, b, recip(b)); }
 // a / b for a value that every thread of the group holds: any operands, the
@@ -1316,7 +1324,7 @@ __device__ __forceinline__ T residual_of(T r, double alpha, T ap) { return (T)((
 template <typename T>
 __device__ __forceinline__ T precond_of(T r, T dg) {
   const double dgd = (double)dg;
-  return (T)((fabs(dgd) > 1e-20) ? div_rn((double)r, dgd) : (double)r);
+  return (T)select(fabs(dgd) > 1e-20, div_rn((double)r, dgd), (double)r);
 }
 
 // Iteration 0 (x0 = 0; p0 = z0, A p0 and p0.A p0 come from phase C): x, and
@@ -1487,7 +1495,7 @@ __device__ __forceinline__ int pcg_tiles(const DesignView& d, Group& g, double* 
       r[k] = residual_of(ro, alpha0, apo);
     }
     const double dgd = (double)dgo;
-    S.inv[k][th] = fabs(dgd) > 1e-20 ? recip(dgd) : 0.0;
+    S.inv[k][th] = select(fabs(dgd) > 1e-20, recip(dgd), 0.0);
     S.z[k][th] = mine ? precond_of(r[k], dgo) : (T)0;
     S.p[k][ip] = mine ? pc : (T)0;
     S.dg[k][th] = dgo;
@@ -1568,7 +1576,7 @@ __device__ __forceinline__ int pcg_tiles(const DesignView& d, Group& g, double* 
       r[k] = residual_of(r[k], alpha, ap[k]);
       const double rr = (double)r[k], y = S.inv[k][th];
       s2[0] += rr * rr;
-      const T z = (T)(__double2hiint(y) != 0 ? div_rn(rr, (double)S.dg[k][th], y) : rr);
+      const T z = (T)select(__double2hiint(y) != 0, div_rn(rr, (double)S.dg[k][th], y), rr);
       S.z[k][th] = z;
       s2[1] += rr * (double)z;
       if (((on >> k) & 1u) && (edge || stored)) {
@@ -1732,6 +1740,234 @@ __device__ __forceinline__ int pcg_stream(const DesignView& d, Group& g, double*
   return it;
 }
 
+// ---------------------------------------------------------------------------
+// The same iterations for a design with one tile per CTA and at most 128 tiles,
+// by the first 16 CTAs alone, which are one thread-block cluster; the other
+// CTAs wait for the outcome at one grid barrier.  On such designs an iteration
+// is two grid reductions of about 1.9 us with 0.6 us of work between them, and
+// a cluster reduces through distributed shared memory in a quarter of that.
+// A warp takes a whole tile: its lanes are the columns, the 8 rows of a column
+// sit in one thread's registers.  Neighbouring tiles push the z of their edges
+// into the tile's ring in shared memory, the tiles' partial sums go to all 16
+// CTAs, and one cluster barrier publishes both.
+// The sums keep the grid's order (32 columns by a xor tree, the 8 rows in
+// order, tile t in lane t mod 32, a xor tree), so the bits are those of
+// pcg_tiles on as many CTAs as tiles.
+// B200, us per outer iteration from zero: 200 x 100 (91 tiles, 20 CG iterations)
+// 112 -> 89, 233 x 61 (64 tiles, 200 CG iterations) 956 -> 592: 2.9 us per CG
+// iteration instead of 4.7.  A single warp per scheduler carries the work, so
+// its instruction latencies bound it (P1 0.5, P2 0.4, the sums and the barrier
+// 2 x 0.9 us).
+// ---------------------------------------------------------------------------
+constexpr int kClusterCtas = 16, kClusterTiles = 128;
+
+template <typename T>
+struct PcgCluster {
+  static constexpr int kRows = 8, kWarps = kThreads / 32;
+  double inv[kRows][kThreads];
+  T x[kRows][kThreads], dg[kRows][kThreads], cW[kRows][kThreads], cE[kRows][kThreads], cN[kRows][kThreads];
+  alignas(16) T ring[kWarps][kHalo];  // z at the tile's south row, north row, west column, east column
+  double part1[kClusterTiles], part2[2][kClusterTiles];
+};
+
+// The sum of a warp's tile in the grid's order; every lane gets it.
+__device__ __forceinline__ double tile_sum(const double (&v)[8]) {
+  const int lane = threadIdx.x & 31;
+  double a[4], b[2], c;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const double got = __shfl_xor_sync(0xffffffffu, (lane & 16) ? v[q] : v[4 + q], 16);
+    a[q] = ((lane & 16) ? v[4 + q] : v[q]) + got;
+  }
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    const double got = __shfl_xor_sync(0xffffffffu, (lane & 8) ? a[q] : a[2 + q], 8);
+    b[q] = ((lane & 8) ? a[2 + q] : a[q]) + got;
+  }
+  {
+    const double got = __shfl_xor_sync(0xffffffffu, (lane & 4) ? b[0] : b[1], 4);
+    c = ((lane & 4) ? b[1] : b[0]) + got;
+  }
+  c += __shfl_xor_sync(0xffffffffu, c, 2);
+  c += __shfl_xor_sync(0xffffffffu, c, 1);
+  // row q is in the lanes 16 (q >> 2) + 8 (q >> 1 & 1) + 4 (q & 1)
+  double row[8];
+#pragma unroll
+  for (int q = 0; q < 8; ++q) row[q] = __shfl_sync(0xffffffffu, c, 16 * (q >> 2) + 8 * ((q >> 1) & 1) + 4 * (q & 1));
+  double s = row[0];
+#pragma unroll
+  for (int q = 1; q < 8; ++q) s += row[q];
+  return s;
+}
+// All tiles' partial sums in the grid's order, two values at a time.
+__device__ __forceinline__ void fold_tiles(const double* p0, const double* p1, int tiles, double& s0, double& s1) {
+  double a = 0.0, b = 0.0;
+#pragma unroll
+  for (int q = 0; q < kClusterTiles / 32; ++q) {
+    const int t = (int)(threadIdx.x & 31) + 32 * q;
+    const double x = t < tiles ? p0[t] : 0.0, y = t < tiles ? p1[t] : 0.0;
+    a += x;
+    b += y;
+  }
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) {
+    a += __shfl_xor_sync(0xffffffffu, a, off);
+    b += __shfl_xor_sync(0xffffffffu, b, off);
+  }
+  s0 = a;
+  s1 = b;
+}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
+template <typename T>
+__device__ __forceinline__ int pcg_cluster(const DesignView& d, int rank, char* tbuf, double alpha0, double rz,
+                                           double beta) {
+  static_assert(sizeof(T) == 0 || (kTileI == 8 && kTileJ == 32), "a warp's tile");
+  using Sm = PcgCluster<T>;
+  constexpr int R = Sm::kRows;
+  Sm& S = *reinterpret_cast<Sm*>(tbuf);
+  cg::cluster_group cl = cg::this_cluster();
+  const Inner<T>& w = inner<T>(d);
+  const int M = d.M, N = d.N, P = d.P;
+  const int tilesJ = (N - 1 + kTileJ - 1) / kTileJ, tiles = tilesJ * ((M - 1 + kTileI - 1) / kTileI);
+  const int th = threadIdx.x, wp = th >> 5, lane = th & 31;
+  const int per = (tiles + kClusterCtas - 1) / kClusterCtas;  // tiles of a CTA
+  const int t = rank * per + wp;
+  const bool works = wp < per && t < tiles;
+  const int ti = t / tilesJ, tj = t - ti * tilesJ, i0 = 1 + ti * kTileI, j = 1 + tj * kTileJ + lane;
+  unsigned on = 0;
+  T r[R], p[R], z[R];
+  T cS0 = (T)0, pS = (T)0, pN = (T)0, pc = (T)0;
+  T* const ring = S.ring[wp < Sm::kWarps ? wp : 0];
+  // where this tile's edge values go: the rings of the neighbouring tiles
+  T *toS = nullptr, *toN = nullptr, *toSide = nullptr;
+  if (works) {
+    auto p0 = [&](int i, int jj) { return w.pp0[i * P + jj]; };
+    auto z1 = [&](int i, int jj) {
+      const int o = i * P + jj;
+      return precond_of(residual_of(w.pr[o], alpha0, w.pAp[o]), w.pdiag[o]);
+    };
+    auto unknown = [&](int i, int jj) { return i >= 1 && i <= M - 1 && jj >= 1 && jj <= N - 2; };
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+      const bool mine = unknown(i0 + q, j);
+      on |= mine ? 1u << q : 0u;
+      const int o = mine ? (i0 + q) * P + j : P + 1;
+      const T ro = w.pr[o], ap = w.pAp[o], xo = w.px[o], po = w.pp0[o], dg = w.pdiag[o], ce = w.cx[o], cn = w.cy[o],
+              cw = w.cx[o - 1];
+      r[q] = mine ? residual_of(ro, alpha0, ap) : (T)0;
+      z[q] = mine ? precond_of(r[q], dg) : (T)0;
+      p[q] = mine ? po : (T)0;
+      S.cE[q][th] = mine ? ce : (T)0;
+      S.cN[q][th] = mine ? cn : (T)0;
+      S.cW[q][th] = (mine && j > 1) ? cw : (T)0;
+      S.x[q][th] = mine ? xo : (T)0;
+      S.dg[q][th] = dg;
+      S.inv[q][th] = select(fabs((double)dg) > 1e-20, recip((double)dg), 0.0);
+    }
+    cS0 = (i0 > 1 && unknown(i0 - 1, j)) ? w.cy[(i0 - 1) * P + j] : (T)0;
+    T zs = (T)0, zn = (T)0, zc = (T)0;
+    if (unknown(i0 - 1, j)) { pS = p0(i0 - 1, j); zs = z1(i0 - 1, j); }
+    if (unknown(i0 + R, j)) { pN = p0(i0 + R, j); zn = z1(i0 + R, j); }
+    ring[lane] = zs;
+    ring[32 + lane] = zn;
+    if (lane < 2 * R) {
+      const int i = i0 + (lane & (R - 1)), jc = lane < R ? j - lane - 1 : j - lane + kTileJ;
+      if (unknown(i, jc)) { pc = p0(i, jc); zc = z1(i, jc); }
+      ring[64 + lane] = zc;
+    }
+    auto ring_of = [&](int tile, int at) {
+      return cl.map_shared_rank(&S.ring[tile % per][at], tile / per);
+    };
+    if (ti > 0) toS = ring_of(t - tilesJ, 32 + lane);
+    if (t + tilesJ < tiles) toN = ring_of(t + tilesJ, lane);
+    if (lane == 0 && tj > 0) toSide = ring_of(t - 1, 64 + R);
+    if (lane == 31 && tj + 1 < tilesJ) toSide = ring_of(t + 1, 64);
+  }
+  double *to1 = nullptr, *to2 = nullptr;  // lane q < 16: this tile's partial sums in CTA q
+  if (works && lane < kClusterCtas) {
+    to1 = cl.map_shared_rank(&S.part1[t], lane);
+    to2 = cl.map_shared_rank(&S.part2[0][t], lane);
+  }
+  __syncwarp();
+  int it = 1;
+  for (; it < d.maxPIter; ++it) {
+    // p = z + beta p (pressure_solver.cpp:181)
+    auto pk = [&](T zq, T pq) -> T { return (T)((double)zq + beta * (double)pq); };
+    if (works) {
+      double v[R], cs = (double)cS0;
+#pragma unroll
+      for (int q = 0; q < R; ++q) p[q] = pk(z[q], p[q]);
+      pS = pk(ring[lane], pS);
+      pN = pk(ring[32 + lane], pN);
+      pc = pk(ring[64 + (lane & (2 * R - 1))], pc);
+#pragma unroll
+      for (int q = 0; q < R; ++q) {
+        const T side = __shfl_sync(0xffffffffu, pc, lane == 31 ? R + q : q);
+        T pw = __shfl_up_sync(0xffffffffu, p[q], 1), pe = __shfl_down_sync(0xffffffffu, p[q], 1);
+        if (lane == 0) pw = side;
+        if (lane == 31) pe = side;
+        const double pq = (double)p[q];
+        double Ap = 0.0;
+        Ap += -cs * (double)(q > 0 ? p[q > 0 ? q - 1 : 0] : pS);
+        Ap += -(double)S.cW[q][th] * (double)pw;
+        Ap += (double)S.dg[q][th] * pq;
+        Ap += -(double)S.cE[q][th] * (double)pe;
+        cs = (double)S.cN[q][th];  // the next row's south conductance
+        Ap += -cs * (double)(q < R - 1 ? p[q < R - 1 ? q + 1 : q] : pN);
+        z[q] = ((on >> q) & 1u) ? (T)Ap : (T)0;  // A p, until z is formed below
+        v[q] = 0.0 + pq * (double)z[q];
+      }
+      const double s = tile_sum(v);
+      if (to1) *to1 = s;
+    }
+    cluster_arrive();
+    cluster_wait();
+    double pAp, unused;
+    fold_tiles(S.part1, S.part1, tiles, pAp, unused);
+    if (fabs(pAp) < 1e-20) break;
+    const double alpha = div_uniform(rz, pAp);
+    if (works) {
+      double vr[R], vz[R];
+#pragma unroll
+      for (int q = 0; q < R; ++q) {
+        r[q] = residual_of(r[q], alpha, z[q]);
+        const double rr = (double)r[q], y = S.inv[q][th];
+        z[q] = (T)select(__double2hiint(y) != 0, div_rn(rr, (double)S.dg[q][th], y), rr);
+        vr[q] = 0.0 + rr * rr;
+        vz[q] = 0.0 + rr * (double)z[q];
+      }
+      if (toS) *toS = z[0];
+      if (toN) *toN = z[R - 1];
+      if (toSide) {
+#pragma unroll
+        for (int q = 0; q < R; ++q) toSide[q] = z[q];
+      }
+      const double s0 = tile_sum(vr), s1 = tile_sum(vz);
+      if (to2) {
+        to2[0] = s0;
+        to2[kClusterTiles] = s1;
+      }
+    }
+    cluster_arrive();
+    if (works) {
+#pragma unroll
+      for (int q = 0; q < R; ++q) S.x[q][th] = (T)((double)S.x[q][th] + alpha * (double)p[q]);
+    }
+    cluster_wait();
+    double rr, rzNew;
+    fold_tiles(S.part2[0], S.part2[1], tiles, rr, rzNew);
+    if (rr < d.pStop) break;
+    beta = div_uniform(rzNew, rz);
+    rz = rzNew;
+  }
+#pragma unroll
+  for (int q = 0; q < R; ++q)
+    if ((on >> q) & 1u) w.px[(i0 + q) * P + j] = S.x[q][th];
+  return it;
+}
+
 inline __host__ __device__ int pcg_tiles_of(int M, int N) {
   return ((M - 1 + kTileI - 1) / kTileI) * ((N - 1 + kTileJ - 1) / kTileJ);
 }
@@ -1767,6 +2003,10 @@ __device__ __forceinline__ int pcg_two_reductions(const DesignView& d, Group& g,
   if (s2[0] < d.pStop) return 0;
   if (d.maxPIter == 1) return 1;
   const double rz = s2[1], beta = div_uniform(rz, rz0);
+  if constexpr (Carry == kCluster) {
+    const int its = g.rank < (unsigned)kClusterCtas ? pcg_cluster<T>(d, (int)g.rank, tbuf, alpha, rz, beta) : 0;
+    return g.sync() ? its : -1;  // the count is CTA 0's to report
+  }
   if constexpr ((Carry & kFew) != 0)
     if ((Carry & kForms) == kFew || form == kFew) return pcg_tiles<T, kFewTiles>(d, g, smem, tbuf, alpha, rz, beta);
   if constexpr ((Carry & kMany) != 0)
@@ -2107,7 +2347,7 @@ __device__ bool mass_phase(const DesignView& d, Group& g, double* smem, char* tb
             double aP = aE + aW + aN + aS;
             if (aP < 1e-20) aP = 1.0;
             const double rr = (double)(T)b, dd = (double)(T)aP;
-            z = (double)(T)((fabs(dd) > 1e-20) ? div_rn(rr, dd) : rr);
+            z = (double)(T)select(fabs(dd) > 1e-20, div_rn(rr, dd), rr);
           }
           z0.ref(k) = z;
         }
@@ -2359,7 +2599,7 @@ __device__ bool dp_phase(const DesignView& d, Group& g, double* smem, char* tbuf
 // Dynamic shared memory a persistent kernel needs for storage type T (the
 // tile buffers).
 template <typename T>
-constexpr size_t tile_smem_bytes() {
+__host__ __device__ constexpr size_t tile_smem_bytes() {
   constexpr size_t a = kStageDepth * LayoutA::kBytes;
   constexpr size_t c = kStageDepth * LayoutC<T>::kBytes + LayoutC<T>::kExtraBytes;
   constexpr size_t dd = kStageDepth * LayoutD<T>::kBytes;
@@ -2373,12 +2613,35 @@ constexpr size_t tile_smem_bytes() {
   return t > q ? t : q;
 }
 
-// The kernels declare their dynamic shared memory (the tile buffers, where
-// TMA tile copies land) 128-byte aligned.  Checked once at the start of a
-// launch: a CTA whose buffer is not aligned records kStatusTimeout (the host
-// reports a failed device wait) and the launch does no work.
-__device__ __forceinline__ bool tile_buffer_aligned(const char* dyn, int* status) {
-  const bool bad = (smem_u32(dyn) & 127u) != 0;
+// Dynamic shared memory of a kernel that carries `Carry`, and of the monitored
+// one, whose pressure-drop windows (window_values doubles at most) use the
+// buffers after phase D.
+template <typename T>
+__host__ __device__ constexpr size_t window_values() {
+  constexpr size_t R = PcgTileCount<T>::value, kM = sizeof(T) == 4 ? R : 1;
+  return sizeof(T) * (kThreads * (6 * R + 2 * kM) + R * (2 * kHalo + kTileI + kTileJ)) / sizeof(double);
+}
+template <typename T, int Carry, bool Monitor>
+__host__ __device__ constexpr size_t kernel_smem_bytes() {
+  // one CTA per SM for the cluster form: its 16 CTAs on 16 SMs, and the other
+  // phases spread as without clusters (packed two to an SM, the late outer
+  // iterations of a 64-tile design took 22.1 instead of 21.1 us)
+  constexpr size_t one = 116 * 1024;
+  static_assert(sizeof(PcgCluster<T>) <= one, "cluster PCG state");
+  constexpr size_t t = tile_smem_bytes<T>(), c = Carry == kCluster ? one : 0;
+  constexpr size_t m = Monitor ? window_values<T>() * sizeof(double) : 0;
+  return t > c ? (t > m ? t : m) : (c > m ? c : m);
+}
+
+// Checked once at the start of a launch: the kernels declare their dynamic
+// shared memory (the tile buffers, where TMA tile copies land) 128-byte
+// aligned, and the launch gives at least `bytes` of it.  A CTA that finds
+// otherwise records kStatusTimeout (the host reports a failed device wait)
+// and the launch does no work.
+__device__ __forceinline__ bool tile_buffer_fits(const char* dyn, size_t bytes, int* status) {
+  unsigned given;
+  asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(given));
+  const bool bad = (smem_u32(dyn) & 127u) != 0 || given < bytes;
   if (bad && threadIdx.x == 0 && status) atomicCAS(status, kStatusOk, kStatusTimeout);
   return !__syncthreads_or(bad);
 }

@@ -10,14 +10,15 @@
 // CFL controllers compiled in (their registers spill the plain kernel's).
 // Carry: the PCG forms and options compiled in (cps::Carries).
 template <typename T, bool Monitor, bool Pseudo, int Carry>
-__global__ void __launch_bounds__(cps::kThreads, CPS_MIN_BLOCKS) cps_grid_kernel(cps::DesignView d, cps::RunControl rc,
+__global__ void __launch_bounds__(cps::kThreads, Carry == cps::kCluster ? 1 : CPS_MIN_BLOCKS) cps_grid_kernel(cps::DesignView d, cps::RunControl rc,
                                                                 cps::GridBarrier* bar, double* red) {
   __shared__ double smem[(Monitor ? cps::kPlaneSums : cps::kRedWidth) * 8];
   __shared__ cps::PseudoRun s_pr;
   __shared__ double out[8];
   extern __shared__ __align__(128) char tile_smem[];
-  cps::GridGroup g{bar, red, rc.status, blockIdx.x, gridDim.x, 0u, 0ull};
-  if (!cps::tile_buffer_aligned(tile_smem, rc.status)) return;
+  if ((int)blockIdx.x >= rc.ctas) return;
+  cps::GridGroup g{bar, red, rc.status, blockIdx.x, (unsigned)rc.ctas, 0u, 0ull};
+  if (!cps::tile_buffer_fits(tile_smem, cps::kernel_smem_bytes<T, Carry, Monitor>(), rc.status)) return;
   cps::tma_barriers_init();
   cps::load_pseudo(d, s_pr);
   __syncthreads();
@@ -50,7 +51,7 @@ __global__ void __launch_bounds__(cps::kThreads) cps_cluster_kernel(const cps::B
   extern __shared__ __align__(128) char tile_smem[];
   cps::cg::cluster_group cl = cps::cg::this_cluster();
   cps::ClusterGroup g{redbuf, nullptr, cl.block_rank(), cl.num_blocks(), 0u};
-  if (!cps::tile_buffer_aligned(tile_smem, &results[0].status)) return;
+  if (!cps::tile_buffer_fits(tile_smem, cps::tile_smem_bytes<T>(), &results[0].status)) return;
   cps::tma_barriers_init();
   for (;;) {
     if (g.rank == 0 && threadIdx.x == 0) s_next = atomicAdd(queue, 1);
@@ -112,7 +113,7 @@ __global__ void __launch_bounds__(cps::kThreads, CPS_MIN_BLOCKS) cps_group_kerne
   int* slot = slots + 2 * grp;  // [0] next queue index, [1] group status before a design is assigned
   cps::GridGroup g{bars + grp, rings + (size_t)grp * cps::kRedSlots * group_ctas * cps::kRedWidth, slot + 1,
                    blockIdx.x % group_ctas, (unsigned)group_ctas, 0u, 0ull};
-  if (!cps::tile_buffer_aligned(tile_smem, &results[0].status)) return;
+  if (!cps::tile_buffer_fits(tile_smem, cps::tile_smem_bytes<T>(), &results[0].status)) return;
   cps::tma_barriers_init();
   for (;;) {
     g.status = slot + 1;
@@ -171,7 +172,7 @@ __global__ void __launch_bounds__(cps::kThreads, CPS_MIN_BLOCKS) cps_wave_kernel
   __shared__ cps::PseudoRun s_pr;
   __shared__ double out[8];
   extern __shared__ __align__(128) char tile_smem[];
-  if (!cps::tile_buffer_aligned(tile_smem, &results[which[0]].status)) return;
+  if (!cps::tile_buffer_fits(tile_smem, cps::tile_smem_bytes<T>(), &results[which[0]].status)) return;
   cps::tma_barriers_init();
   int lo = 0, hi = groups;  // first[lo] <= blockIdx.x < first[lo + 1]
   while (hi - lo > 1) {
@@ -221,7 +222,13 @@ __global__ void __launch_bounds__(cps::kThreads, CPS_MIN_BLOCKS) cps_wave_kernel
 #define CPS_GRID_KERNELS(PRE, T)                                                                                    \
   CPS_GRID_KERNEL(PRE, T, false, false, cps::kFew)                                                                  \
   CPS_GRID_KERNEL(PRE, T, false, false, cps::kMany)                                                                 \
-  CPS_GRID_KERNEL(PRE, T, false, false, cps::kLarge)
+  CPS_GRID_KERNEL(PRE, T, false, false, cps::kLarge)                                                                \
+  CPS_GRID_CLUSTER_KERNELS(PRE, T)
+#if CPS_TILE_J == 32  // the cluster form is written for 8 x 32 tiles
+#define CPS_GRID_CLUSTER_KERNELS(PRE, T) CPS_GRID_KERNEL(PRE, T, false, false, cps::kCluster)
+#else
+#define CPS_GRID_CLUSTER_KERNELS(PRE, T)
+#endif
 #define CPS_GRID_OPTION_KERNELS(PRE, T)                                                                             \
   CPS_GRID_KERNEL(PRE, T, false, true, cps::kAll)                                                                   \
   CPS_GRID_KERNEL(PRE, T, true, true, cps::kAll)

@@ -68,6 +68,7 @@ __global__ void __launch_bounds__(cps::kThreads, CPS_MIN_BLOCKS) cps_noalloc_ker
   __shared__ double out[8];
   extern __shared__ __align__(128) char tile_smem[];
   cps::GridGroup g{bar, red, rc.status, blockIdx.x, gridDim.x, 0u, 0ull};  // no tensor maps: element-wise staging
+  if (!cps::tile_buffer_fits(tile_smem, cps::tile_smem_bytes<double>(), rc.status)) return;
   cps::SweepHint hint{2, 2};
   for (int it = 0; it < rc.n_outer; ++it) {
     const int r = cps::outer_iteration<double>(d, g, smem, tile_smem, out, it + 1 == rc.n_outer,
