@@ -626,6 +626,35 @@ __global__ void __launch_bounds__(cps::kThreads) cps_barrier_selftest_kernel(cps
   g.sync();
 }
 
+namespace {
+
+// The batch kernels of a storage type, by what their designs need.
+struct BatchKernels {
+  const void *cluster, *group, *wave;
+};
+template <typename T, bool Options, int Carry>
+BatchKernels batch_kernels() {
+  return {(const void*)cps_cluster_kernel<T, Options, Carry>, (const void*)cps_group_kernel<T, Options, Carry>,
+          (const void*)cps_wave_kernel<T, Options, Carry>};
+}
+// ctas[k]: the CTAs of design k.  pcg_tiles<many> serves the designs of few
+// tiles too: carrying one form costs them less than carrying two (group kernel
+// with both: 84 bytes of spills, with the larger one 4).
+template <typename T>
+BatchKernels batch_kernels(cps_ctx* const* ctxs, const std::vector<int>& ctas, bool options) {
+  if (options) return batch_kernels<T, true, cps::kAll>();
+  int most = cps::kFew;
+  for (size_t k = 0; k < ctas.size(); ++k) most = std::max(most, cps::pcg_form<T>(ctxs[k]->M, ctxs[k]->N, ctas[k]));
+  if (most == cps::kFew) return batch_kernels<T, false, cps::kFew>();
+  return most == cps::kMany ? batch_kernels<T, false, cps::kMany>() : batch_kernels<T, false, cps::kForms>();
+}
+BatchKernels batch_kernels(cps_ctx* const* ctxs, const std::vector<int>& ctas, bool options) {
+  return ctxs[0]->precision == CPS_MIXED ? batch_kernels<float>(ctxs, ctas, options)
+                                         : batch_kernels<double>(ctxs, ctas, options);
+}
+
+}  // namespace
+
 extern "C" {
 
 const char* cps_version(void) { return "cps 0.2 (sm_100a)"; }
@@ -1103,9 +1132,8 @@ cps_status cps_batch_solve(cps_ctx* const* ctxs, int n, const double* inletVeloc
   if (opts->tiles_per_cta > 0) {
     // Groups sized to their designs, packed into waves (first fit, largest
     // first); one cooperative launch per wave, all CTAs of a wave co-resident.
-    const void* wk = c0->precision == CPS_MIXED
-                         ? (options ? (const void*)cps_wave_kernel<float, true> : (const void*)cps_wave_kernel<float, false>)
-                         : (options ? (const void*)cps_wave_kernel<double, true> : (const void*)cps_wave_kernel<double, false>);
+    // (every batch kernel fits the SM as often as every other: they share the shared memory and launch bounds)
+    const void* wk = batch_kernels(ctxs, {}, options).wave;
     int per_sm = 0, sms = 0;
     const size_t tsm = tile_smem_for(c0->precision);
     if (!allow_smem(c0, wk, tsm) ||
@@ -1120,6 +1148,8 @@ cps_status cps_batch_solve(cps_ctx* const* ctxs, int n, const double* inletVeloc
                               ((ctxs[k]->N - 1 + cps::kTileJ - 1) / cps::kTileJ);
       ctas[k] = (int)std::max(1LL, std::min<long long>(max_ctas, (tiles + opts->tiles_per_cta - 1) / opts->tiles_per_cta));
     }
+    wk = batch_kernels(ctxs, ctas, options).wave;
+    if (!allow_smem(c0, wk, tsm)) return CPS_ERR_CUDA;
     std::vector<int> byc(n);
     std::iota(byc.begin(), byc.end(), 0);
     std::stable_sort(byc.begin(), byc.end(), [&](int a, int b) { return ctas[a] > ctas[b]; });
@@ -1164,9 +1194,7 @@ cps_status cps_batch_solve(cps_ctx* const* ctxs, int n, const double* inletVeloc
     }
   } else if (opts->group_ctas > 0) {
     // Groups of CTAs in one cooperative launch (all CTAs co-resident).
-    const void* gk = c0->precision == CPS_MIXED
-                         ? (options ? (const void*)cps_group_kernel<float, true> : (const void*)cps_group_kernel<float, false>)
-                         : (options ? (const void*)cps_group_kernel<double, true> : (const void*)cps_group_kernel<double, false>);
+    const void* gk = batch_kernels(ctxs, std::vector<int>(n, opts->group_ctas), options).group;
     int per_sm = 0, sms = 0;
     const size_t tsm = tile_smem_for(c0->precision);
     if (!allow_smem(c0, gk, tsm) ||
@@ -1193,14 +1221,11 @@ cps_status cps_batch_solve(cps_ctx* const* ctxs, int n, const double* inletVeloc
                  "cooperative group launch"))
       return CPS_ERR_CUDA;
   } else {
-  using KernFn = void (*)(const cps::BatchItem*, const int*, int, int*, cps::BatchResult*);
-  KernFn kern = c0->precision == CPS_MIXED
-                    ? (options ? (KernFn)cps_cluster_kernel<float, true> : (KernFn)cps_cluster_kernel<float, false>)
-                    : (options ? (KernFn)cps_cluster_kernel<double, true> : (KernFn)cps_cluster_kernel<double, false>);
+  const void* kern = batch_kernels(ctxs, std::vector<int>(n, cl), options).cluster;
   if (cl > 8 &&
-      !cuda_ok(c0, cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1), "attr"))
+      !cuda_ok(c0, cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1), "attr"))
     return CPS_ERR_CUDA;
-  if (!allow_smem(c0, (const void*)kern, tile_smem_for(c0->precision))) return CPS_ERR_CUDA;
+  if (!allow_smem(c0, kern, tile_smem_for(c0->precision))) return CPS_ERR_CUDA;
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -1214,7 +1239,7 @@ cps_status cps_batch_solve(cps_ctx* const* ctxs, int n, const double* inletVeloc
   cfg.numAttrs = 1;
   cfg.gridDim = dim3(cl * 64);
   int max_clusters = 0;
-  if (!cuda_ok(c0, cudaOccupancyMaxActiveClusters(&max_clusters, (const void*)kern, &cfg), "cluster occupancy"))
+  if (!cuda_ok(c0, cudaOccupancyMaxActiveClusters(&max_clusters, kern, &cfg), "cluster occupancy"))
     return CPS_ERR_CUDA;
   if (max_clusters < 1) return fail(c0, CPS_ERR_CUDA, "cluster configuration does not fit");
   int clusters = std::min(max_clusters, n);
@@ -1225,7 +1250,8 @@ cps_status cps_batch_solve(cps_ctx* const* ctxs, int n, const double* inletVeloc
   int* queue = ws->queue;
   cps::BatchResult* res = ws->results;
   if (!cuda_ok(c0, cudaEventRecord(ws->ev0, st), "event")) return CPS_ERR_CUDA;
-  if (!cuda_ok(c0, cudaLaunchKernelEx(&cfg, kern, items, order, n, queue, res), "cluster launch")) return CPS_ERR_CUDA;
+  void* args[] = {&items, &order, &n, &queue, &res};
+  if (!cuda_ok(c0, cudaLaunchKernelExC(&cfg, kern, args), "cluster launch")) return CPS_ERR_CUDA;
   }
   if (!cuda_ok(c0, cudaEventRecord(ws->ev1, st), "event") ||
       !cuda_ok(c0, cudaMemcpyAsync(ws->h_results, ws->results, sizeof(cps::BatchResult) * n, cudaMemcpyDeviceToHost,

@@ -38,7 +38,7 @@ __global__ void __launch_bounds__(cps::kThreads, Carry == cps::kCluster ? 1 : CP
 
 // Batched solves: each cluster takes the next design from the queue and runs
 // its outer iterations to convergence or to the item's budget.
-template <typename T, bool Options>
+template <typename T, bool Options, int Carry>
 __global__ void __launch_bounds__(cps::kThreads) cps_cluster_kernel(const cps::BatchItem* __restrict__ items,
                                                                    const int* __restrict__ order, int n_items,
                                                                    int* queue, cps::BatchResult* results) {
@@ -74,7 +74,7 @@ __global__ void __launch_bounds__(cps::kThreads) cps_cluster_kernel(const cps::B
     int done = 0;
     cps::SweepHint hint{2, 2};
     for (int it = 0; it < item.n_outer; ++it) {
-      const int r = cps::outer_iteration<T, cps::ClusterGroup, false, Options, Options ? cps::kAll : cps::kForms>(
+      const int r = cps::outer_iteration<T, cps::ClusterGroup, false, Options, Carry>(
           item.view, g, smem, tile_smem, out, it + 1 == item.n_outer, item.stop_on_conv != 0, item.eps, item.iter0 + it,
           nullptr, nullptr, &s_pr, &hint);
       done = it + 1;
@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(cps::kThreads) cps_cluster_kernel(const cps::B
 // time and runs each with the bounded software barrier of its own counter.
 // The group count sets how many designs are in flight (and so the in-flight
 // working set against the 126 MB L2); K sets how many CTAs share one design.
-template <typename T, bool Options>
+template <typename T, bool Options, int Carry>
 __global__ void __launch_bounds__(cps::kThreads, CPS_MIN_BLOCKS) cps_group_kernel(const cps::BatchItem* __restrict__ items,
                                                                     const int* __restrict__ order, int n_items,
                                                                     int* queue, cps::BatchResult* results,
@@ -138,7 +138,7 @@ __global__ void __launch_bounds__(cps::kThreads, CPS_MIN_BLOCKS) cps_group_kerne
     int done = 0;
     cps::SweepHint hint{2, 2};
     for (int it = 0; it < item.n_outer; ++it) {
-      const int r = cps::outer_iteration<T, cps::GridGroup, false, Options, Options ? cps::kAll : cps::kForms>(
+      const int r = cps::outer_iteration<T, cps::GridGroup, false, Options, Carry>(
           item.view, g, smem, tile_smem, out, it + 1 == item.n_outer, item.stop_on_conv != 0, item.eps, item.iter0 + it,
           nullptr, nullptr, &s_pr, &hint);
       if (r < 0) return;  // a bounded wait expired; the design's status says so
@@ -161,7 +161,7 @@ __global__ void __launch_bounds__(cps::kThreads, CPS_MIN_BLOCKS) cps_group_kerne
 // designs.  CTAs [first[g], first[g+1]) form group g and run design which[g]
 // to convergence or to its budget with the bounded software barrier of their
 // own counter; their reduction ring starts at first[g] ring rows.
-template <typename T, bool Options>
+template <typename T, bool Options, int Carry>
 __global__ void __launch_bounds__(cps::kThreads, CPS_MIN_BLOCKS) cps_wave_kernel(const cps::BatchItem* __restrict__ items,
                                                                    const int* __restrict__ first,
                                                                    const int* __restrict__ which, int groups,
@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(cps::kThreads, CPS_MIN_BLOCKS) cps_wave_kernel
   int done = 0;
   cps::SweepHint hint{2, 2};
   for (int it = 0; it < item.n_outer; ++it) {
-    const int r = cps::outer_iteration<T, cps::GridGroup, false, Options, Options ? cps::kAll : cps::kForms>(
+    const int r = cps::outer_iteration<T, cps::GridGroup, false, Options, Carry>(
         item.view, g, smem, tile_smem, out, it + 1 == item.n_outer, item.stop_on_conv != 0, item.eps, item.iter0 + it,
         nullptr, nullptr, &s_pr, &hint);
     if (r < 0) return;  // a bounded wait expired; the design's status says so
@@ -213,9 +213,10 @@ __global__ void __launch_bounds__(cps::kThreads, CPS_MIN_BLOCKS) cps_wave_kernel
   }
 }
 
-// Every instantiation the library launches, storage type T.  Batches carry all
-// PCG forms (their designs differ in size); Options adds the pseudo-transient
-// term, the CFL controllers and the options of cps::kOptions.
+// Every instantiation the library launches, storage type T.  A batch carries
+// the on-chip PCG form its designs need, all forms when one of them needs more
+// (kForms), and with Options the pseudo-transient term, the CFL controllers
+// and the options of cps::kOptions too.
 #define CPS_GRID_KERNEL(PRE, T, MONITOR, PSEUDO, CARRY)                                                             \
   PRE template __global__ void cps_grid_kernel<T, MONITOR, PSEUDO, CARRY>(cps::DesignView, cps::RunControl,         \
                                                                           cps::GridBarrier*, double*);
@@ -232,13 +233,16 @@ __global__ void __launch_bounds__(cps::kThreads, CPS_MIN_BLOCKS) cps_wave_kernel
 #define CPS_GRID_OPTION_KERNELS(PRE, T)                                                                             \
   CPS_GRID_KERNEL(PRE, T, false, true, cps::kAll)                                                                   \
   CPS_GRID_KERNEL(PRE, T, true, true, cps::kAll)
-#define CPS_BATCH_KERNELS_OF(PRE, T, OPTIONS)                                                                       \
-  PRE template __global__ void cps_cluster_kernel<T, OPTIONS>(const cps::BatchItem*, const int*, int, int*,          \
-                                                              cps::BatchResult*);                                   \
-  PRE template __global__ void cps_group_kernel<T, OPTIONS>(const cps::BatchItem*, const int*, int, int*,            \
-                                                            cps::BatchResult*, cps::GridBarrier*, double*, int*,    \
-                                                            int);                                                   \
-  PRE template __global__ void cps_wave_kernel<T, OPTIONS>(const cps::BatchItem*, const int*, const int*, int,        \
-                                                           cps::BatchResult*, cps::GridBarrier*, double*);
-#define CPS_BATCH_KERNELS(PRE, T) CPS_BATCH_KERNELS_OF(PRE, T, false)
-#define CPS_BATCH_OPTION_KERNELS(PRE, T) CPS_BATCH_KERNELS_OF(PRE, T, true)
+#define CPS_BATCH_KERNELS_OF(PRE, T, OPTIONS, CARRY)                                                                \
+  PRE template __global__ void cps_cluster_kernel<T, OPTIONS, CARRY>(const cps::BatchItem*, const int*, int, int*,  \
+                                                                     cps::BatchResult*);                            \
+  PRE template __global__ void cps_group_kernel<T, OPTIONS, CARRY>(const cps::BatchItem*, const int*, int, int*,    \
+                                                                   cps::BatchResult*, cps::GridBarrier*, double*,   \
+                                                                   int*, int);                                      \
+  PRE template __global__ void cps_wave_kernel<T, OPTIONS, CARRY>(const cps::BatchItem*, const int*, const int*,    \
+                                                                  int, cps::BatchResult*, cps::GridBarrier*, double*);
+#define CPS_BATCH_KERNELS(PRE, T)                                                                                   \
+  CPS_BATCH_KERNELS_OF(PRE, T, false, cps::kFew)                                                                    \
+  CPS_BATCH_KERNELS_OF(PRE, T, false, cps::kMany)                                                                   \
+  CPS_BATCH_KERNELS_OF(PRE, T, false, cps::kForms)
+#define CPS_BATCH_OPTION_KERNELS(PRE, T) CPS_BATCH_KERNELS_OF(PRE, T, true, cps::kAll)
