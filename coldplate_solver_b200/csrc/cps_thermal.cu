@@ -38,8 +38,34 @@ constexpr int kMaxNz = 64;
 constexpr int kMaxCtas = 2048;
 enum Plane { kW = 0, kE, kS, kN, kB, kT, kD };
 
+// Exact n / d for 0 <= n < 2^31 by a multiplication (Granlund and Montgomery,
+// "Division by invariant integers using multiplication", 1994): a cell's
+// indices cost a few instructions instead of two integer divisions.
+struct FastDiv {
+  unsigned mul, shift;
+  int d;
+  static FastDiv of(int d) {
+    FastDiv f{0, 0, d};
+    while ((1u << (f.shift + 1)) <= (unsigned)d) ++f.shift;
+    if ((1u << f.shift) == (unsigned)d) {  // n >> 1 by the multiplication, the rest by the shift
+      f.mul = 1u << 31;
+      f.shift = f.shift > 0 ? f.shift - 1 : 0;
+    } else {
+      f.mul = (unsigned)((1ull << (32 + f.shift)) / (unsigned)d + 1ull);
+    }
+    return f;
+  }
+  __device__ __forceinline__ int operator()(int n) const { return d == 1 ? n : (int)(__umulhi((unsigned)n, mul) >> shift); }
+};
+
+// x0 and x1 (and level 0's iterates) have a layer of zeros before and after
+// them: with A's entries zero where a neighbour does not exist, the stencil
+// reads all seven places without conditions.
 struct Level {
   int nx, ny, nz, n;
+  FastDiv dnx, dplane;
+  int cstride;     // values between A's planes in global memory
+  int lx0, lx1, lb, lc;  // levels run by one CTA: offsets in its shared memory (lc < 0: A stays in global memory)
   double* c[7];    // W E S N B T diagonal
   double* x0;      // iterate / correction (coarse levels)
   double* x1;      // Jacobi partner
@@ -48,6 +74,8 @@ struct Level {
 
 struct View {
   int nlev, maxiter, sweeps;
+  int split;                  // levels [split, nlev) run in CTA 0's shared memory
+  int lfactor;                // offset of the coarsest column's factors there (2 nz values)
   double rtol, omega, alpha;
   Level lv[kMaxLevels];
   double *rhs, *T, *r, *rhat, *p, *v, *s, *t;  // level-0 Krylov vectors
@@ -212,19 +240,22 @@ __global__ void coarsen_kernel(Level F, Level C) {
   }
 }
 
-// (A x)[P] on level L, the entries in CSR column order.
-__device__ __forceinline__ double apply(const Level& L, const double* __restrict__ x, int P) {
-  const int nx = L.nx, plane = L.nx * L.ny;
-  const int i = P % nx, j = (P / nx) % L.ny, k = P / plane;
+// (A x)[P], the entries in CSR column order; stride n between A's planes.
+__device__ __forceinline__ double stencil(double cB, double cS, double cW, double cD, double cE, double cN, double cT,
+                                          const double* x, int nx, int plane) {
   double s = 0.0;
-  if (k > 0) s += L.c[kB][P] * x[P - plane];
-  if (j > 0) s += L.c[kS][P] * x[P - nx];
-  if (i > 0) s += L.c[kW][P] * x[P - 1];
-  s += L.c[kD][P] * x[P];
-  if (i < nx - 1) s += L.c[kE][P] * x[P + 1];
-  if (j < L.ny - 1) s += L.c[kN][P] * x[P + nx];
-  if (k < L.nz - 1) s += L.c[kT][P] * x[P + plane];
+  s += cB * x[-plane];
+  s += cS * x[-nx];
+  s += cW * x[-1];
+  s += cD * x[0];
+  s += cE * x[1];
+  s += cN * x[nx];
+  s += cT * x[plane];
   return s;
+}
+__device__ __forceinline__ double apply(const Level& L, const double* __restrict__ x, int P) {
+  return stencil(L.c[kB][P], L.c[kS][P], L.c[kW][P], L.c[kD][P], L.c[kE][P], L.c[kN][P], L.c[kT][P], x + P, L.nx,
+                 L.dplane.d);
 }
 
 struct Loop {
@@ -232,151 +263,235 @@ struct Loop {
   __device__ Loop() : start(blockIdx.x * blockDim.x + threadIdx.x), stride(gridDim.x * blockDim.x) {}
 };
 
-// Levels with at most this many cells run inside CTA 0 alone (block-stride
-// loops, CTA barriers): below it a grid barrier costs more than the work.
+// ---------------------------------------------------------------------------
+// The coarsest levels, by CTA 0 in its shared memory: below a few thousand
+// cells a grid barrier costs more than the work, and out of global memory the
+// phases of these levels took 20 to 45 us of a V-cycle, a memory latency each
+// (250 x 125 x 9, five levels: 45 -> 18 us).
+// Iterates, right-hand sides and the small levels' coefficients live in shared
+// memory for the whole solve; load_local fills it once per launch.
+// ---------------------------------------------------------------------------
+constexpr size_t kLocalSmem = 52 * 1024;  // per CTA: three CTAs per SM keep 60 KB of L1
 constexpr int kLocalCells = 2048;
 
-// Where a phase runs: the whole grid (grid-stride loops, grid barrier) or,
-// with Local, CTA 0 alone (block-stride loops, __syncthreads).
-template <bool Local>
-struct Exec {
-  int start, stride;
-  cps::GridGroup* g;
-  __device__ explicit Exec(cps::GridGroup* gg) : g(gg) {
-    start = Local ? (int)threadIdx.x : (int)(blockIdx.x * blockDim.x + threadIdx.x);
-    stride = Local ? (int)blockDim.x : (int)(gridDim.x * blockDim.x);
+__device__ __forceinline__ void load_local(const View& tv, double* sm) {
+  const int last = tv.nlev - 1, th = threadIdx.x;
+  for (int l = tv.split; l <= last; ++l) {
+    const Level& L = tv.lv[l];
+    const int pad = L.dplane.d;
+    for (int q = th; q < L.n + 2 * pad; q += cps::kThreads) sm[L.lx0 - pad + q] = sm[L.lx1 - pad + q] = 0.0;
+    if (L.lc >= 0)
+      for (int p = 0; p < 7; ++p)
+        for (int P = th; P < L.n; P += cps::kThreads) sm[L.lc + p * L.n + P] = L.c[p][P];
   }
-  __device__ bool sync() {
-    if (Local) {
-      __syncthreads();
-      return true;
+  if (th == 0) {
+    // the tridiagonal factors of the coarsest column (Thomas algorithm)
+    const Level& Z = tv.lv[last];
+    double *cp = sm + tv.lfactor, *m = cp + Z.nz;
+    for (int k = 0; k < Z.nz; ++k) {
+      const double a = k > 0 ? Z.c[kB][k] : 0.0;
+      m[k] = Z.c[kD][k] - (k > 0 ? a * cp[k - 1] : 0.0);
+      cp[k] = cps::div_rn(Z.c[kT][k], m[k]);
     }
-    return g->sync();
+  }
+  __syncthreads();
+}
+
+// A level in shared memory, its places in registers: read through the View in
+// the loops they would be loaded again after every store.
+struct LocalLevel {
+  int n, nx, ny, plane, cs;
+  const double* c;  // A's planes, cs values apart (in shared memory, or global for the larger levels)
+  double *x0, *x1, *b;
+  __device__ __forceinline__ LocalLevel(const Level& L, double* sm)
+      : n(L.n), nx(L.nx), ny(L.ny), plane(L.dplane.d), cs(L.lc >= 0 ? L.n : L.cstride),
+        c(L.lc >= 0 ? sm + L.lc : L.c[0]), x0(sm + L.lx0), x1(sm + L.lx1), b(sm + L.lb) {}
+  // (A x)[P]; the diagonal entry too
+  __device__ __forceinline__ double mul(const double* x, int P, double& cD) const {
+    const double* q = c + P;
+    cD = q[kD * cs];
+    return stencil(q[kB * cs], q[kS * cs], q[kW * cs], cD, q[kE * cs], q[kN * cs], q[kT * cs], x + P, nx, plane);
   }
 };
 
-// The first level at or below which every level is small enough for CTA 0.
-__device__ __forceinline__ int local_from(const View& tv) {
-  int l = tv.nlev - 1;
-  while (l > 0 && tv.lv[l - 1].n <= kLocalCells) --l;
-  return l;
+// One V-cycle over levels [split, nlev) on rhs (level split); its result goes to out.
+__device__ __forceinline__ void local_vcycle(const View& tv, const double* __restrict__ rhs, double* __restrict__ out,
+                                             double* sm) {
+  const int last = tv.nlev - 1, th = threadIdx.x, first = tv.split, sweeps = tv.sweeps;
+  const double w = tv.omega, alpha = tv.alpha;
+  {
+    const LocalLevel L(tv.lv[first], sm);
+    for (int P = th; P < L.n; P += cps::kThreads) L.b[P] = rhs[P];
+  }
+  // xo = xi + w (b - A xi) / D
+  auto sweep = [w, th](const LocalLevel& L, const double* xi, double* xo) {
+#pragma unroll 4
+    for (int P = th; P < L.n; P += cps::kThreads) {
+      double cD;
+      const double s = L.mul(xi, P, cD);
+      xo[P] = xi[P] + cps::div_rn(w * (L.b[P] - s), cD);
+    }
+    __syncthreads();
+  };
+  __syncthreads();
+  for (int l = first; l < last; ++l) {
+    const LocalLevel L(tv.lv[l], sm);
+    const FastDiv dnx = tv.lv[l + 1].dnx, dplane = tv.lv[l + 1].dplane;
+    const int cn = tv.lv[l + 1].n;
+    double* cb = sm + tv.lv[l + 1].lb;
+    for (int P = th; P < L.n; P += cps::kThreads) L.x0[P] = cps::div_rn(w * L.b[P], L.c[P + kD * L.cs]);
+    __syncthreads();
+    double *xa = L.x0, *xb = L.x1;
+    for (int sw = 1; sw < sweeps; ++sw) {
+      sweep(L, xa, xb);
+      double* t = xa; xa = xb; xb = t;
+    }
+    // the residual into the free iterate, then its sums over the aggregates
+#pragma unroll 4
+    for (int P = th; P < L.n; P += cps::kThreads) {
+      double cD;
+      xb[P] = L.b[P] - L.mul(xa, P, cD);
+    }
+    __syncthreads();
+    for (int Q = th; Q < cn; Q += cps::kThreads) {
+      const int k = dplane(Q), r = Q - k * dplane.d, J = dnx(r), I = r - J * dnx.d;
+      const double* f = xb + k * L.plane + 2 * J * L.nx + 2 * I;
+      const bool e = 2 * I + 1 < L.nx, nn = 2 * J + 1 < L.ny;
+      double acc = 0.0 + f[0];
+      if (e) acc += f[1];
+      if (nn) acc += f[L.nx];
+      if (e && nn) acc += f[L.nx + 1];
+      cb[Q] = acc;
+    }
+    __syncthreads();
+  }
+  double* x = sm + tv.lv[last].lx0;
+  {
+    const LocalLevel Z(tv.lv[last], sm);
+    if (th == 0) {
+      const double *cp = sm + tv.lfactor, *m = cp + Z.n;
+      double prev = 0.0;
+      for (int k = 0; k < Z.n; ++k) {
+        const double a = k > 0 ? Z.c[k + kB * Z.cs] : 0.0;
+        prev = cps::div_rn(Z.b[k] - (k > 0 ? a * prev : 0.0), m[k]);
+        x[k] = prev;
+      }
+      for (int k = Z.n - 2; k >= 0; --k) x[k] = x[k] - cp[k] * x[k + 1];
+    }
+    __syncthreads();
+  }
+  for (int l = last - 1; l >= first; --l) {
+    const LocalLevel L(tv.lv[l], sm);
+    const FastDiv dnx = tv.lv[l].dnx, dplane = tv.lv[l].dplane;
+    const int cnx = tv.lv[l + 1].nx, cplane = tv.lv[l + 1].dplane.d;
+    double *xa = ((sweeps - 1) & 1) ? L.x1 : L.x0, *xb = xa == L.x0 ? L.x1 : L.x0;
+    for (int P = th; P < L.n; P += cps::kThreads) {
+      const int k = dplane(P), r = P - k * dplane.d, j = dnx(r), i = r - j * dnx.d;
+      xa[P] += alpha * x[k * cplane + (j >> 1) * cnx + (i >> 1)];
+    }
+    __syncthreads();
+    for (int sw = 0; sw < sweeps; ++sw) {
+      sweep(L, xa, xb);
+      double* t = xa; xa = xb; xb = t;
+    }
+    x = xa;
+  }
+  const int n = tv.lv[first].n;
+  for (int P = th; P < n; P += cps::kThreads) out[P] = x[P];
 }
 
-// One V-cycle over levels [l0, nlev) on rhs0 (level l0), iterate buffers
-// a0/a1 of level l0.  Every non-coarsest level's result ends in its second
-// buffer (2 sweeps - 1 swaps in all), the coarsest's in its first; so the
-// caller knows where the result is without being told.  The grid instance
-// hands the small levels to CTA 0 and waits at one grid barrier.
-template <bool Local>
-__device__ double* vcycle_from(const View& tv, cps::GridGroup& g, int l0, const double* rhs0, double* a0, double* a1,
-                               bool& ok) {
-  Exec<Local> ex(&g);
-  double* cur[kMaxLevels];
-  double* oth[kMaxLevels];
-  const double w = tv.omega;
-  const double* rhs = rhs0;
-  const int last = tv.nlev - 1;
-  const int split = Local ? last + 1 : local_from(tv);  // grid instance: levels >= split go to CTA 0
-  int l = l0;
-  for (; l < last && (Local || l < split); ++l) {
+// ---------------------------------------------------------------------------
+// One V-cycle on level 0's right-hand side rhs0 with iterate buffers a0, a1;
+// returns its result (one of them).  The caller has formed the first sweep,
+// x = w rhs / D, into a0 together with rhs; on the coarser levels the thread
+// that forms a right-hand side forms its first sweep too, so that a level
+// takes 2 sweeps grid phases on the way down and up together with its
+// restriction instead of 2 sweeps + 1.  What bounds it: on the finest level of
+// a large case HBM (1000 x 500 x 9, 80 bytes per cell and phase at 5.5 TB/s),
+// below about 100 k cells the grid barrier, 1.7 us beside 1 to 2 us of work.
+// B200, ms per solve with five phases per level, index divisions in the
+// stencil and the small levels out of global memory -> now: 100 x 40 x 9
+// 2.9 -> 1.9, 250 x 125 x 9 8.7 -> 5.4, 500 x 240 x 9 23.2 -> 16.0,
+// 1000 x 500 x 9 95 -> 80.
+// ---------------------------------------------------------------------------
+__device__ double* vcycle(const View& tv, cps::GridGroup& g, const double* rhs0, double* a0, double* a1, double* sm,
+                          bool& ok) {
+  const Loop lp;
+  const double w = tv.omega, alpha = tv.alpha;
+  const int split = tv.split, sweeps = tv.sweeps;
+  if (split == 0) {
+    if (g.rank == 0) local_vcycle(tv, rhs0, a1, sm);
+    if (!g.sync()) ok = false;
+    return a1;
+  }
+  for (int l = 0; l < split; ++l) {
     const Level& L = tv.lv[l];
-    double* xa = l == l0 ? a0 : L.x0;
-    double* xb = l == l0 ? a1 : L.x1;
-    for (int P = ex.start; P < L.n; P += ex.stride) xa[P] = w * rhs[P] / L.c[kD][P];
-    if (!ex.sync()) { ok = false; return a0; }
-    for (int sw = 1; sw < tv.sweeps; ++sw) {
-      for (int P = ex.start; P < L.n; P += ex.stride) xb[P] = xa[P] + w * (rhs[P] - apply(L, xa, P)) / L.c[kD][P];
-      double* tmp = xa; xa = xb; xb = tmp;
-      if (!ex.sync()) { ok = false; return a0; }
-    }
     const Level& C = tv.lv[l + 1];
-    const int fplane = L.nx * L.ny, cplane = C.nx * C.ny;
-    for (int Q = ex.start; Q < C.n; Q += ex.stride) {
-      const int I = Q % C.nx, J = (Q / C.nx) % C.ny, k = Q / cplane;
-      double acc = 0.0;
-      for (int bb = 0; bb < 2; ++bb)
-        for (int aa = 0; aa < 2; ++aa) {
-          const int i = 2 * I + aa, j = 2 * J + bb;
-          if (i >= L.nx || j >= L.ny) continue;
-          const int f = k * fplane + j * L.nx + i;
-          acc += rhs[f] - apply(L, xa, f);
-        }
-      C.b[Q] = acc;
+    const double* rhs = l ? L.b : rhs0;
+    double *xa = l ? L.x0 : a0, *xb = l ? L.x1 : a1;
+    for (int sw = 1; sw < sweeps; ++sw) {
+      for (int P = lp.start; P < L.n; P += lp.stride)
+        xb[P] = xa[P] + cps::div_rn(w * (rhs[P] - apply(L, xa, P)), L.c[kD][P]);
+      double* tmp = xa; xa = xb; xb = tmp;
+      if (!g.sync()) { ok = false; return a0; }
     }
-    if (!ex.sync()) { ok = false; return a0; }
-    cur[l] = xa;
-    oth[l] = xb;
-    rhs = C.b;
-  }
-  // l is now the first level this instance does not descend from
-  if (!Local && l < last) {
-    // levels [l, last] inside CTA 0; the rest of the grid waits at the barrier
-    double* x0 = l == l0 ? a0 : tv.lv[l].x0;
-    double* x1 = l == l0 ? a1 : tv.lv[l].x1;
-    if (g.rank == 0) vcycle_from<true>(tv, g, l, rhs, x0, x1, ok);
-    if (!g.sync()) { ok = false; return a0; }
-    cur[l] = x1;
-  } else {
-    // coarsest: one column of nz cells, tridiagonal in z (Thomas algorithm)
-    const Level& Z = tv.lv[last];
-    double* xz = last == l0 ? a0 : Z.x0;
-    if ((Local || g.rank == 0) && threadIdx.x == 0) {
-      double cp[kMaxNz], dp[kMaxNz];
-      const int nz = Z.nz;
-      for (int k = 0; k < nz; ++k) {
-        const double a = k > 0 ? Z.c[kB][k] : 0.0;
-        const double m = Z.c[kD][k] - (k > 0 ? a * cp[k - 1] : 0.0);
-        cp[k] = Z.c[kT][k] / m;
-        dp[k] = (rhs[k] - (k > 0 ? a * dp[k - 1] : 0.0)) / m;
+    const int plane = L.dplane.d;
+    const bool first = l + 1 < split;  // the next level's first sweep
+    // four lanes to a coarse cell, one per fine cell of its aggregate
+    for (int q = lp.start; q < ((4 * C.n + 31) & ~31); q += lp.stride) {
+      const int Q = q >> 2, k = C.dplane(Q), r = Q - k * C.dplane.d, J = C.dnx(r), I = r - J * C.nx;
+      const int i = 2 * I + (q & 1), j = 2 * J + ((q >> 1) & 1), f = k * plane + j * L.nx + i;
+      double res = 0.0;
+      if (Q < C.n && i < L.nx && j < L.ny) res = rhs[f] - apply(L, xa, f);
+      const double r1 = __shfl_down_sync(0xffffffffu, res, 1), r2 = __shfl_down_sync(0xffffffffu, res, 2),
+                   r3 = __shfl_down_sync(0xffffffffu, res, 3);
+      if ((q & 3) == 0 && Q < C.n) {
+        const double acc = 0.0 + res + r1 + r2 + r3;  // cells beyond the edge count 0
+        C.b[Q] = acc;
+        if (first) C.x0[Q] = cps::div_rn(w * acc, C.c[kD][Q]);
       }
-      xz[nz - 1] = dp[nz - 1];
-      for (int k = nz - 2; k >= 0; --k) xz[k] = dp[k] - cp[k] * xz[k + 1];
     }
-    if (!ex.sync()) { ok = false; return a0; }
-    cur[last] = xz;
-    l = last;
+    if (!g.sync()) { ok = false; return a0; }
   }
-  for (int m = l - 1; m >= l0; --m) {
-    const Level& L = tv.lv[m];
-    const Level& C = tv.lv[m + 1];
-    const double* rhsl = m == l0 ? rhs0 : L.b;
-    double* xa = cur[m];
-    double* xb = oth[m];
-    const double* e = cur[m + 1];
-    const int fplane = L.nx * L.ny, cplane = C.nx * C.ny;
-    const double alpha = tv.alpha;
+  if (g.rank == 0) local_vcycle(tv, tv.lv[split].b, tv.lv[split].x1, sm);
+  if (!g.sync()) { ok = false; return a0; }
+  const double* e = tv.lv[split].x1;
+  for (int l = split - 1; l >= 0; --l) {
+    const Level& L = tv.lv[l];
+    const Level& C = tv.lv[l + 1];
+    const double* rhs = l ? L.b : rhs0;
+    double *x0 = l ? L.x0 : a0, *x1 = l ? L.x1 : a1;
+    double *xa = ((sweeps - 1) & 1) ? x1 : x0, *xb = xa == x0 ? x1 : x0;
+    const int nx = L.nx, ny = L.ny, nz = L.nz, plane = L.dplane.d, cnx = C.nx, cplane = C.dplane.d;
     // First post-smoothing sweep with the coarse correction folded in: every
-    // value it reads is x + alpha e(parent), computed as the separate
+    // value it reads is x + alpha e(parent), computed as a separate
     // prolongation pass would have stored it (the same operations, so the same
     // bits), which saves that pass and its barrier.
-    for (int P = ex.start; P < L.n; P += ex.stride) {
-      const int i = P % L.nx, j = (P / L.nx) % L.ny, k = P / fplane;
-      auto xc = [&](int q, int ii, int jj, int kk) { return xa[q] + alpha * e[kk * cplane + (jj >> 1) * C.nx + (ii >> 1)]; };
+    for (int P = lp.start; P < L.n; P += lp.stride) {
+      const int k = L.dplane(P), r = P - k * plane, j = L.dnx(r), i = r - j * nx;
+      auto xc = [&](int q, int ii, int jj, int kk) { return xa[q] + alpha * e[kk * cplane + (jj >> 1) * cnx + (ii >> 1)]; };
       double s = 0.0;  // A x in apply()'s order
-      if (k > 0) s += L.c[kB][P] * xc(P - fplane, i, j, k - 1);
-      if (j > 0) s += L.c[kS][P] * xc(P - L.nx, i, j - 1, k);
+      if (k > 0) s += L.c[kB][P] * xc(P - plane, i, j, k - 1);
+      if (j > 0) s += L.c[kS][P] * xc(P - nx, i, j - 1, k);
       if (i > 0) s += L.c[kW][P] * xc(P - 1, i - 1, j, k);
-      const double xP = xc(P, i, j, k);
-      s += L.c[kD][P] * xP;
-      if (i < L.nx - 1) s += L.c[kE][P] * xc(P + 1, i + 1, j, k);
-      if (j < L.ny - 1) s += L.c[kN][P] * xc(P + L.nx, i, j + 1, k);
-      if (k < L.nz - 1) s += L.c[kT][P] * xc(P + fplane, i, j, k + 1);
-      xb[P] = xP + w * (rhsl[P] - s) / L.c[kD][P];
+      const double xP = xc(P, i, j, k), cD = L.c[kD][P];
+      s += cD * xP;
+      if (i < nx - 1) s += L.c[kE][P] * xc(P + 1, i + 1, j, k);
+      if (j < ny - 1) s += L.c[kN][P] * xc(P + nx, i, j + 1, k);
+      if (k < nz - 1) s += L.c[kT][P] * xc(P + plane, i, j, k + 1);
+      xb[P] = xP + cps::div_rn(w * (rhs[P] - s), cD);
     }
     { double* tmp = xa; xa = xb; xb = tmp; }
-    if (!ex.sync()) { ok = false; return a0; }
-    for (int sw = 1; sw < tv.sweeps; ++sw) {
-      for (int P = ex.start; P < L.n; P += ex.stride) xb[P] = xa[P] + w * (rhsl[P] - apply(L, xa, P)) / L.c[kD][P];
+    if (!g.sync()) { ok = false; return a0; }
+    for (int sw = 1; sw < sweeps; ++sw) {
+      for (int P = lp.start; P < L.n; P += lp.stride)
+        xb[P] = xa[P] + cps::div_rn(w * (rhs[P] - apply(L, xa, P)), L.c[kD][P]);
       double* tmp = xa; xa = xb; xb = tmp;
-      if (!ex.sync()) { ok = false; return a0; }
+      if (!g.sync()) { ok = false; return a0; }
     }
-    cur[m] = xa;
+    e = xa;
   }
-  return cur[l0];
-}
-
-__device__ double* vcycle(const View& tv, cps::GridGroup& g, const double* rhs0, double* a0, double* a1, bool& ok) {
-  return vcycle_from<false>(tv, g, 0, rhs0, a0, a1, ok);
+  return const_cast<double*>(e);
 }
 
 // BiCGStab, right-preconditioned by the V-cycle, from T = T_inlet.
@@ -387,10 +502,12 @@ __device__ double* vcycle(const View& tv, cps::GridGroup& g, const double* rhs0,
 #ifndef CPT_MIN_BLOCKS
 #define CPT_MIN_BLOCKS 3
 #endif
-__global__ void __launch_bounds__(cps::kThreads, CPT_MIN_BLOCKS) solve_kernel(View tv, double T_in, int warm, cps::GridBarrier* bar,
+__global__ void __launch_bounds__(cps::kThreads, CPT_MIN_BLOCKS) solve_kernel(const __grid_constant__ View tv, double T_in, int warm, cps::GridBarrier* bar,
                                                                  double* red, int* status) {
   __shared__ double smem[cps::kRedWidth * 8];
+  extern __shared__ __align__(16) double local_sm[];
   cps::GridGroup g{bar, red, status, blockIdx.x, gridDim.x, 0u, 0ull};
+  if (g.rank == 0) load_local(tv, local_sm);
   const Loop lp;
   const Level& L = tv.lv[0];
   const int n = L.n;
@@ -417,9 +534,13 @@ __global__ void __launch_bounds__(cps::kThreads, CPT_MIN_BLOCKS) solve_kernel(Vi
   bool conv = sqrt(rr) <= tv.rtol * bnorm;
   while (!conv && it < tv.maxiter) {
     const double beta = (rho_new / rho) * (alpha / omega);
-    for (int P = lp.start; P < n; P += lp.stride) tv.p[P] = tv.r[P] + beta * (tv.p[P] - omega * tv.v[P]);
+    for (int P = lp.start; P < n; P += lp.stride) {
+      const double pv = tv.r[P] + beta * (tv.p[P] - omega * tv.v[P]);
+      tv.p[P] = pv;
+      tv.ph0[P] = cps::div_rn(tv.omega * pv, L.c[kD][P]);  // the V-cycle's first sweep
+    }
     if (!g.sync()) return;
-    double* ph = vcycle(tv, g, tv.p, tv.ph0, tv.ph1, ok);
+    double* ph = vcycle(tv, g, tv.p, tv.ph0, tv.ph1, local_sm, ok);
     if (!ok) return;
     double q1[1] = {0.0};
     for (int P = lp.start; P < n; P += lp.stride) {
@@ -433,6 +554,7 @@ __global__ void __launch_bounds__(cps::kThreads, CPT_MIN_BLOCKS) solve_kernel(Vi
     for (int P = lp.start; P < n; P += lp.stride) {
       const double s = tv.r[P] - alpha * tv.v[P];
       tv.s[P] = s;
+      tv.sh0[P] = cps::div_rn(tv.omega * s, L.c[kD][P]);
       qs[0] += s * s;
     }
     if (!g.sync_reduce<1, 0u>(qs, smem)) return;
@@ -443,7 +565,7 @@ __global__ void __launch_bounds__(cps::kThreads, CPT_MIN_BLOCKS) solve_kernel(Vi
       conv = true;
       break;
     }
-    double* sh = vcycle(tv, g, tv.s, tv.sh0, tv.sh1, ok);
+    double* sh = vcycle(tv, g, tv.s, tv.sh0, tv.sh1, local_sm, ok);
     if (!ok) return;
     double q3[2] = {0.0, 0.0};
     for (int P = lp.start; P < n; P += lp.stride) {
@@ -520,6 +642,33 @@ bool tcuda(cps_thermal* t, cudaError_t e, const char* what) {
   if (e == cudaSuccess) return true;
   tfail(t, CPS_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
   return false;
+}
+
+// The levels CTA 0 runs alone and where it keeps them in its shared memory:
+// from the coarsest up, as long as a level has at most kLocalCells cells and
+// iterates and right-hand sides fit; then the coefficients of the smallest
+// levels in what is left.  The coarsest column (at most 64 cells) always fits.
+void plan_local(cpt::View& tv) {
+  const size_t room = cpt::kLocalSmem / sizeof(double);
+  const cpt::Level& Z = tv.lv[tv.nlev - 1];
+  size_t used = 2 * (size_t)Z.nz;
+  tv.lfactor = 0;
+  int l = tv.nlev - 1;
+  for (; l >= 0; --l) {
+    cpt::Level& L = tv.lv[l];
+    const size_t pad = L.dplane.d, need = 3 * (size_t)L.n + 4 * pad;
+    if (L.n > cpt::kLocalCells || used + need > room) break;
+    L.lx0 = (int)(used + pad);
+    L.lx1 = L.lx0 + L.n + 2 * (int)pad;
+    L.lb = L.lx1 + L.n + (int)pad;
+    L.lc = -1;
+    used += need;
+  }
+  tv.split = l + 1;
+  for (l = tv.nlev - 1; l >= tv.split && used + 7 * (size_t)tv.lv[l].n <= room; --l) {
+    tv.lv[l].lc = (int)used;
+    used += 7 * (size_t)tv.lv[l].n;
+  }
 }
 
 // Upload the 2-D inputs (q0 NULL: the uniform flux) and assemble level 0 and
@@ -606,6 +755,8 @@ cps_status cps_thermal_create(const cps_thermal_desc* d, cps_thermal** out) {
       L.ny = ny;
       L.nz = Nz;
       L.n = nx * ny * Nz;
+      L.dnx = cpt::FastDiv::of(nx);
+      L.dplane = cpt::FastDiv::of(nx * ny);
       if (nx == 1 && ny == 1) break;
       nx = (nx + 1) / 2;
       ny = (ny + 1) / 2;
@@ -613,8 +764,9 @@ cps_status cps_thermal_create(const cps_thermal_desc* d, cps_thermal** out) {
   }
   const size_t n0 = (size_t)tv.lv[0].n, n2 = (size_t)d->Nx * d->Ny;
   auto al = [](size_t elems) { return (elems * sizeof(double) + 255) / 256 * 256; };
-  size_t bytes = al(n0) * (7 + 1 + 1 + 6 + 4);
-  for (int l = 1; l < tv.nlev; ++l) bytes += al(tv.lv[l].n) * 10;
+  auto padded = [&](int l) { return (size_t)tv.lv[l].n + 2 * (size_t)tv.lv[l].dplane.d; };  // iterates: a layer around
+  size_t bytes = al(n0) * (7 + 1 + 6) + al(padded(0)) * 5;
+  for (int l = 1; l < tv.nlev; ++l) bytes += al(tv.lv[l].n) * 8 + al(padded(l)) * 2;
   bytes += al(n2) * 4 + 256 + al((size_t)cps::kRedSlots * cps::kRedWidth * cpt::kMaxCtas) + 256;
   if (!tcuda(t, cudaSetDevice(d->device), "cudaSetDevice") ||
       !tcuda(t, cudaStreamCreateWithFlags(&t->stream, cudaStreamNonBlocking), "stream"))
@@ -630,25 +782,28 @@ cps_status cps_thermal_create(const cps_thermal_desc* d, cps_thermal** out) {
     cur += al(elems);
     return p;
   };
+  auto take_iterate = [&](int l) { return take(padded(l)) + tv.lv[l].dplane.d; };
   for (int p = 0; p < 7; ++p) tv.lv[0].c[p] = take(n0);
+  tv.lv[0].cstride = (int)(tv.lv[0].c[1] - tv.lv[0].c[0]);
   tv.rhs = take(n0);
-  tv.T = take(n0);
+  tv.T = take_iterate(0);
   tv.r = take(n0);
   tv.rhat = take(n0);
   tv.p = take(n0);
   tv.v = take(n0);
   tv.s = take(n0);
   tv.t = take(n0);
-  tv.ph0 = take(n0);
-  tv.ph1 = take(n0);
-  tv.sh0 = take(n0);
-  tv.sh1 = take(n0);
+  tv.ph0 = take_iterate(0);
+  tv.ph1 = take_iterate(0);
+  tv.sh0 = take_iterate(0);
+  tv.sh1 = take_iterate(0);
   tv.lv[0].x0 = tv.lv[0].x1 = tv.lv[0].b = nullptr;
   for (int l = 1; l < tv.nlev; ++l) {
     cpt::Level& L = tv.lv[l];
     for (int p = 0; p < 7; ++p) L.c[p] = take(L.n);
-    L.x0 = take(L.n);
-    L.x1 = take(L.n);
+    L.cstride = (int)(L.c[1] - L.c[0]);
+    L.x0 = take_iterate(l);
+    L.x1 = take_iterate(l);
     L.b = take(L.n);
   }
   t->dgamma = take(n2);
@@ -695,8 +850,11 @@ cps_status cps_thermal_create(const cps_thermal_desc* d, cps_thermal** out) {
   const cps_status st = assemble(t, d->gamma, d->u, d->v, d->q0);
   if (st != CPS_OK) return bail(st);
   int per_sm = 0, sms = 0;
-  if (!tcuda(t, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)cpt::solve_kernel, cps::kThreads, 0),
-             "occupancy") ||
+  plan_local(tv);
+  if (!tcuda(t, cudaFuncSetAttribute((const void*)cpt::solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)cpt::kLocalSmem), "smem attribute") ||
+      !tcuda(t, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)cpt::solve_kernel, cps::kThreads,
+                                                              cpt::kLocalSmem), "occupancy") ||
       !tcuda(t, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, d->device), "attribute"))
     return bail(CPS_ERR_CUDA);
   if (per_sm < 1) return bail(tfail(t, CPS_ERR_CUDA, "solve kernel does not fit on an SM"));
@@ -723,8 +881,8 @@ cps_status solve_launch(cps_thermal* t, int warm, cps_thermal_result* res) {
   double T_in = t->desc.T_inlet;
   void* args[] = {&tv, &T_in, &warm, &t->bar, &t->red, &t->status};
   if (!tcuda(t, cudaEventRecord(t->ev0, t->stream), "event") ||
-      !tcuda(t, cudaLaunchCooperativeKernel((const void*)cpt::solve_kernel, dim3(t->grid), dim3(cps::kThreads), args, 0,
-                                            t->stream), "cooperative launch") ||
+      !tcuda(t, cudaLaunchCooperativeKernel((const void*)cpt::solve_kernel, dim3(t->grid), dim3(cps::kThreads), args,
+                                            cpt::kLocalSmem, t->stream), "cooperative launch") ||
       !tcuda(t, cudaEventRecord(t->ev1, t->stream), "event") ||
       !tcuda(t, cudaMemcpyAsync(t->hout, tv.out, 4 * sizeof(double), cudaMemcpyDeviceToHost, t->stream), "d2h") ||
       !tcuda(t, cudaMemcpyAsync(t->hout + 4, t->status, sizeof(int), cudaMemcpyDeviceToHost, t->stream), "d2h") ||
