@@ -1286,26 +1286,44 @@ __device__ __forceinline__ double sweep_point_staged(const DesignView& d, const 
   return r * r;
 }
 
+// One unknown's row, source and iterate, loaded together.  (Rows and columns
+// next to the unknowns exist in every plane; their values are not used.)
+template <typename T>
+struct SweepIn {
+  T cS, cW, cP, cE, cN, b, xS, xW, x, xE, xN;
+};
+
+template <bool IsU, typename T>
+__device__ __forceinline__ SweepIn<T> sweep_load(const DesignView& d, int i, int j, const T* __restrict__ xin) {
+  const Inner<T>& w = inner<T>(d);
+  const T* __restrict__ c = IsU ? w.cU : w.cV;
+  const long long ps = d.planeStride;
+  const int P = d.P;
+  const size_t o = (size_t)i * P + j;
+  return SweepIn<T>{c[o + 3 * ps], c[o + ps], c[o + 4 * ps], c[o], c[o + 2 * ps], (IsU ? w.bU : w.bV)[o],
+                    xin[o - P], xin[o - 1], xin[o], xin[o + 1], xin[o + P]};
+}
+
+template <bool IsU, typename T>
+__device__ __forceinline__ double sweep_point(const DesignView& d, int i, int j, const SweepIn<T>& v,
+                                              T* __restrict__ xout) {
+  const int iHi = IsU ? d.M - 1 : d.M - 2, jHi = IsU ? d.N - 2 : d.N - 1;
+  double Ax = 0.0;
+  if (i - 1 >= 1) Ax += (double)v.cS * (double)v.xS;
+  if (j - 1 >= 1) Ax += (double)v.cW * (double)v.xW;
+  const double aP = (double)v.cP;
+  const double x0 = (double)v.x;
+  Ax += aP * x0;
+  if (j + 1 <= jHi) Ax += (double)v.cE * (double)v.xE;
+  if (i + 1 <= iHi) Ax += (double)v.cN * (double)v.xN;
+  const double r = (double)v.b - Ax;
+  xout[(size_t)i * d.P + j] = (T)(x0 + div_rn(r, aP));
+  return r * r;
+}
 template <bool IsU, typename T>
 __device__ __forceinline__ double sweep_point(const DesignView& d, int i, int j, const T* __restrict__ xin,
                                               T* __restrict__ xout) {
-  const Inner<T>& w = inner<T>(d);
-  const int M = d.M, N = d.N, P = d.P;
-  const int iHi = IsU ? M - 1 : M - 2, jHi = IsU ? N - 2 : N - 1;
-  const T* __restrict__ c = IsU ? w.cU : w.cV;
-  const long long ps = d.planeStride;
-  const size_t o = (size_t)i * P + j;
-  double Ax = 0.0;
-  if (i - 1 >= 1) Ax += (double)c[o + 3 * ps] * (double)xin[o - P];
-  if (j - 1 >= 1) Ax += (double)c[o + ps] * (double)xin[o - 1];
-  const double aP = (double)c[o + 4 * ps];
-  const double x0 = (double)xin[o];
-  Ax += aP * x0;
-  if (j + 1 <= jHi) Ax += (double)c[o] * (double)xin[o + 1];
-  if (i + 1 <= iHi) Ax += (double)c[o + 2 * ps] * (double)xin[o + P];
-  const double r = (double)(IsU ? w.bU : w.bV)[o] - Ax;
-  xout[o] = (T)(x0 + div_rn(r, aP));
-  return r * r;
+  return sweep_point<IsU, T>(d, i, j, sweep_load<IsU, T>(d, i, j, xin), xout);
 }
 
 // x = 0 for phase D, when the PCG stops before its first update.
@@ -1331,25 +1349,42 @@ __device__ __forceinline__ T precond_of(T r, T dg) {
 // |r|^2 and r.z in s2.  Late in a solve it is the only one, so r and z are
 // stored only for the form that reads them back (Store); pcg_tiles forms them
 // again from the same planes.
-template <typename T, bool Store, class Group>
+template <typename T, bool Store, int kU, class Group>
 __device__ __forceinline__ bool pcg_first(const DesignView& d, Group& g, double* smem, double alpha, double (&s2)[2]) {
   const Inner<T>& w = inner<T>(d);
   const int N = d.N, P = d.P;
-  for_each_point(d, g.rank, g.nblk, [&](int i, int j) {
-    if (j > N - 2) return;
-    const size_t o = (size_t)i * P + j;
-    const T pc = w.pp0[o], ro = w.pr[o], ap = w.pAp[o], dg = w.pdiag[o];
-    w.px[o] = (T)(0.0 + alpha * (double)pc);
-    const T rt = residual_of(ro, alpha, ap);
-    const T z = precond_of(rt, dg);
-    if (Store) {
-      w.pr[o] = rt;
-      w.pz[o] = z;
+  // kU tiles' loads before the first of their stores (places beyond the tiles
+  // read a point that exists and leave it)
+  const int M = d.M, tilesJ = (N - 1 + kTileJ - 1) / kTileJ, nt = tilesJ * ((M - 1 + kTileI - 1) / kTileI);
+  const int ty = (int)threadIdx.x / kTileJ, tx = (int)threadIdx.x % kTileJ;
+  for (int t0 = (int)g.rank; t0 < nt; t0 += kU * (int)g.nblk) {
+    int o[kU];
+    T pc[kU], ro[kU], ap[kU], dg[kU];
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      const int t = t0 + u * (int)g.nblk, i = 1 + (t / tilesJ) * kTileI + ty, j = 1 + (t % tilesJ) * kTileJ + tx;
+      o[u] = t < nt && i <= M - 1 && j <= N - 2 ? i * P + j : 0;
+      const int q = o[u] ? o[u] : P + 1;
+      pc[u] = w.pp0[q];
+      ro[u] = w.pr[q];
+      ap[u] = w.pAp[q];
+      dg[u] = w.pdiag[q];
     }
-    const double r = (double)rt;
-    s2[0] += r * r;
-    s2[1] += r * (double)z;
-  });
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      if (!o[u]) continue;
+      w.px[o[u]] = (T)(0.0 + alpha * (double)pc[u]);
+      const T rt = residual_of(ro[u], alpha, ap[u]);
+      const T z = precond_of(rt, dg[u]);
+      if (Store) {
+        w.pr[o[u]] = rt;
+        w.pz[o[u]] = z;
+      }
+      const double r = (double)rt;
+      s2[0] += r * r;
+      s2[1] += r * (double)z;
+    }
+  }
   return g.template sync_reduce<2, 0u>(s2, smem);
 }
 
@@ -1996,9 +2031,11 @@ __device__ __forceinline__ int pcg_two_reductions(const DesignView& d, Group& g,
   const double alpha = div_uniform(rz0, pAp0);
   double s2[2] = {0.0, 0.0};
   bool ok;
-  if constexpr ((Carry & kLarge) == 0) ok = pcg_first<T, false>(d, g, smem, alpha, s2);
-  else if constexpr ((Carry & kForms) == kLarge) ok = pcg_first<T, true>(d, g, smem, alpha, s2);
-  else ok = form == kLarge ? pcg_first<T, true>(d, g, smem, alpha, s2) : pcg_first<T, false>(d, g, smem, alpha, s2);
+  if constexpr (Carry == kCluster) ok = pcg_first<T, false, 1>(d, g, smem, alpha, s2);
+  else if constexpr (Carry == kFew) ok = pcg_first<T, false, kFewTiles>(d, g, smem, alpha, s2);
+  else if constexpr ((Carry & kLarge) == 0) ok = pcg_first<T, false, 4>(d, g, smem, alpha, s2);
+  else if constexpr ((Carry & kForms) == kLarge) ok = pcg_first<T, true, 4>(d, g, smem, alpha, s2);
+  else ok = form == kLarge ? pcg_first<T, true, 4>(d, g, smem, alpha, s2) : pcg_first<T, false, 4>(d, g, smem, alpha, s2);
   if (!ok) return -1;
   if (s2[0] < d.pStop) return 0;
   if (d.maxPIter == 1) return 1;
@@ -2769,10 +2806,19 @@ __device__ int outer_iteration(const DesignView& d, Group& g, double* smem, char
             if (av && i <= M - 2) s[1] += sweep_point_staged<false, T>(d, L, i, j, xoutV);
           });
     } else {
-      for_each_point(d, g.rank, g.nblk, [&](int i, int j) {
-        if (au && j <= N - 2) s[0] += sweep_point<true, T>(d, i, j, xinU, xoutU);
-        if (av && i <= M - 2) s[1] += sweep_point<false, T>(d, i, j, xinV, xoutV);
-      });
+      if (au && av) {
+        // both components' loads before the first store: one memory latency per tile instead of two
+        for_each_point(d, g.rank, g.nblk, [&](int i, int j) {
+          const SweepIn<T> u = sweep_load<true, T>(d, i, j, xinU), v = sweep_load<false, T>(d, i, j, xinV);
+          if (j <= N - 2) s[0] += sweep_point<true, T>(d, i, j, u, xoutU);
+          if (i <= M - 2) s[1] += sweep_point<false, T>(d, i, j, v, xoutV);
+        });
+      } else {
+        for_each_point(d, g.rank, g.nblk, [&](int i, int j) {
+          if (au && j <= N - 2) s[0] += sweep_point<true, T>(d, i, j, xinU, xoutU);
+          if (av && i <= M - 2) s[1] += sweep_point<false, T>(d, i, j, xinV, xoutV);
+        });
+      }
     }
     if (!okB || !g.template sync_reduce<2, 0u>(s, smem)) return -1;
     if (au) { kU = k; actU = !(s[0] < d.thrU) && kU < d.maxMomIter; }
