@@ -44,6 +44,7 @@ NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
     "-lineinfo", "-O3", "--fmad=false", "-std=c++17",
     "-Xcompiler", "-fPIC", "-shared",
+    "-static-global-template-stub=false",  # kernels are instantiated in files of their own
 ]
 
 

@@ -45,6 +45,8 @@ constexpr int kHistChunk = 4096;  // outer iterations per launch inside cps_solv
 constexpr int kFieldPlanes = 10;  // FP64 planes: u v p pc us vs dE dN alpha gamma
 constexpr int kInnerPlanes = 25;  // cU x5, cV x5, bU bV xU0 xU1 xV0 xV1 px pr pz pp0 pp1 pAp pdiag cx cy
 constexpr int kMaxGridCtas = 2048;
+// A context's scratch: the barrier, the flags, the history (bytes from its start), then the rest.
+constexpr size_t kFlagsAt = 64, kHistAt = 256;
 
 enum FieldPlane { kU, kV, kP, kPc, kUs, kVs, kDE, kDN, kAlpha, kGamma };
 
@@ -66,10 +68,14 @@ struct cps_ctx {
   int* dstatus = nullptr;
   int* dndone = nullptr;
   double* dhist = nullptr;
-  double* dplane = nullptr;
   double* hstage = nullptr;  // pinned, one plane of (M+1) x (N+1) doubles
-  double* hhist = nullptr;   // pinned, kHistChunk * 8
-  int* hflags = nullptr;     // pinned: status, n_done, pressure-drop gate
+  // The flags (status, n_done, pressure-drop gate) and the history lie one after
+  // the other on the device and in one pinned buffer, so that a launch's outcome
+  // is one copy.  A plane's metrics are written to the pinned buffer's end by
+  // the kernel itself.
+  int* hflags = nullptr;
+  double* hhist = nullptr;   // kHistChunk * 8
+  double* hplane = nullptr;  // 8
   double* dplog = nullptr;   // device, kHistChunk x 4 pressure drops of the last launch
   double* hdplog = nullptr;  // pinned copy
   double* ddphist = nullptr; // device, the pressure-drop gate's windows (cudaMalloc'd by cps_set_dp_monitor)
@@ -512,21 +518,19 @@ cps_status run(cps_ctx* c, int n_outer, int stop_on_conv, double eps, cps_step_o
     }
     cps::RunControl rc{chunk, stop_on_conv, eps, c->dhist, c->dndone, c->dstatus, c->iter,
                        monitor ? c->dplog : nullptr, c->dstatus + 2, c->grid};
-    if (!cuda_ok(c, cudaMemsetAsync(c->dndone, 0, 2 * sizeof(int), c->stream), "memset") ||
-        !cuda_ok(c, cudaMemsetAsync(c->bar, 0, sizeof(cps::GridBarrier), c->stream), "memset"))
+    // the barrier and the flags
+    if (!cuda_ok(c, cudaMemsetAsync(c->bar, 0, kFlagsAt + 4 * sizeof(int), c->stream), "memset"))
       return CPS_ERR_CUDA;
     void* args[] = {&c->view, &rc, &c->bar, &c->red};
     if (!cuda_ok(c, cudaEventRecord(c->ev0, c->stream), "event")) return CPS_ERR_CUDA;
     if (!cuda_ok(c, launch_grid(c, args), "cooperative launch")) return CPS_ERR_CUDA;
     if (!cuda_ok(c, cudaEventRecord(c->ev1, c->stream), "event")) return CPS_ERR_CUDA;
-    if (!cuda_ok(c, cudaMemcpyAsync(c->hflags, c->dstatus, 3 * sizeof(int), cudaMemcpyDeviceToHost, c->stream), "d2h"))
-      return CPS_ERR_CUDA;
     if (monitor && dp_history &&
         !cuda_ok(c, cudaMemcpyAsync(c->hdplog, c->dplog, sizeof(double) * 4 * chunk, cudaMemcpyDeviceToHost,
                                     c->stream), "d2h"))
       return CPS_ERR_CUDA;
-    if (!cuda_ok(c, cudaMemcpyAsync(c->hhist, c->dhist, sizeof(double) * 8 * chunk, cudaMemcpyDeviceToHost, c->stream),
-                 "d2h"))
+    if (!cuda_ok(c, cudaMemcpyAsync(c->hflags, c->dstatus, kHistAt - kFlagsAt + sizeof(double) * 8 * chunk,
+                                    cudaMemcpyDeviceToHost, c->stream), "d2h"))
       return CPS_ERR_CUDA;
     if (!cuda_ok(c, cudaStreamSynchronize(c->stream), "kernel")) return CPS_ERR_CUDA;
     const int status = c->hflags[0], nd = c->hflags[1];
@@ -739,20 +743,21 @@ cps_status cps_create(const cps_desc* d, cps_ctx** out) {
     return bail(CPS_ERR_CUDA);
   const size_t stage = (size_t)(d->M + 1) * (d->N + 1);
   if (!cuda_ok(c, cudaMallocHost(&c->hstage, stage * sizeof(double)), "pinned alloc") ||
-      !cuda_ok(c, cudaMallocHost(&c->hhist, (size_t)kHistChunk * 8 * sizeof(double)), "pinned alloc") ||
-      !cuda_ok(c, cudaMallocHost(&c->hflags, 4 * sizeof(int)), "pinned alloc") ||
+      !cuda_ok(c, cudaMallocHost(&c->hflags, kHistAt - kFlagsAt + ((size_t)kHistChunk + 1) * 8 * sizeof(double)),
+               "pinned alloc") ||
       !cuda_ok(c, cudaMallocHost(&c->hdplog, sizeof(double) * 4 * kHistChunk), "pinned alloc"))
     return bail(CPS_ERR_OOM);
 
   char* tail = c->slab + c->plane_elems * sizeof(double) * kFieldPlanes +
                round_up(c->plane_elems * elem_bytes(d->precision) * kInnerPlanes, 256);
+  c->hhist = reinterpret_cast<double*>(reinterpret_cast<char*>(c->hflags) + (kHistAt - kFlagsAt));
+  c->hplane = c->hhist + (size_t)kHistChunk * 8;
   c->bar = reinterpret_cast<cps::GridBarrier*>(tail);
-  c->dstatus = reinterpret_cast<int*>(tail + 64);  // [0] status, [1] n_done
+  c->dstatus = reinterpret_cast<int*>(tail + kFlagsAt);  // [0] status, [1] n_done
   c->dndone = c->dstatus + 1;
-  c->red = reinterpret_cast<double*>(tail + 256);
-  c->dhist = c->red + (size_t)(cps::kRedSlots * cps::kRedWidth + cps::kPlaneSums) * kMaxGridCtas;
-  c->dplane = c->dhist + (size_t)kHistChunk * 8;
-  c->dplog = c->dplane + 8;
+  c->dhist = reinterpret_cast<double*>(tail + kHistAt);
+  c->red = c->dhist + (size_t)kHistChunk * 8;
+  c->dplog = c->red + (size_t)(cps::kRedSlots * cps::kRedWidth + cps::kPlaneSums) * kMaxGridCtas + 8;
   c->dpseudo = c->dplog + (size_t)4 * kHistChunk;
   c->dtmaps = reinterpret_cast<cps::TensorMap*>(round_up(reinterpret_cast<size_t>(c->dpseudo + 8), 128));
 
@@ -835,7 +840,6 @@ void cps_destroy(cps_ctx* c) {
   if (c->stream) cudaStreamSynchronize(c->stream);
   if (c->slab) cudaFree(c->slab);
   if (c->hstage) cudaFreeHost(c->hstage);
-  if (c->hhist) cudaFreeHost(c->hhist);
   if (c->hflags) cudaFreeHost(c->hflags);
   if (c->hdplog) cudaFreeHost(c->hdplog);
   if (c->ddphist) cudaFree(c->ddphist);
@@ -1299,13 +1303,11 @@ cps_status cps_get_history(cps_ctx* c, int n, cps_step_out* history) {
 cps_status cps_sample_plane(cps_ctx* c, double x, cps_plane* out) {
   if (!c || !out) return fail(c, CPS_ERR_ARG, "ctx and out are required");
   if (!cuda_ok(c, cudaSetDevice(c->device), "cudaSetDevice")) return CPS_ERR_CUDA;
-  cps_plane_kernel<<<1, cps::kThreads, 0, c->stream>>>(c->view, x, c->dplane);
-  if (!cuda_ok(c, cudaGetLastError(), "plane launch")) return CPS_ERR_CUDA;
-  if (!cuda_ok(c, cudaMemcpyAsync(c->hhist, c->dplane, 6 * sizeof(double), cudaMemcpyDeviceToHost, c->stream), "d2h") ||
-      !cuda_ok(c, cudaStreamSynchronize(c->stream), "plane"))
+  cps_plane_kernel<<<1, cps::kThreads, 0, c->stream>>>(c->view, x, c->hplane);
+  if (!cuda_ok(c, cudaGetLastError(), "plane launch") || !cuda_ok(c, cudaStreamSynchronize(c->stream), "plane"))
     return CPS_ERR_CUDA;
-  out->flowArea = c->hhist[0]; out->massFlux = c->hhist[1]; out->avgStatic = c->hhist[2];
-  out->avgDynamic = c->hhist[3]; out->avgTotal = c->hhist[4]; out->valid = c->hhist[5] != 0.0;
+  out->flowArea = c->hplane[0]; out->massFlux = c->hplane[1]; out->avgStatic = c->hplane[2];
+  out->avgDynamic = c->hplane[3]; out->avgTotal = c->hplane[4]; out->valid = c->hplane[5] != 0.0;
   return CPS_OK;
 }
 
