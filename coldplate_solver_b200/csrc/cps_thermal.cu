@@ -437,18 +437,34 @@ __device__ double* vcycle(const View& tv, cps::GridGroup& g, const double* rhs0,
     }
     const int plane = L.dplane.d;
     const bool first = l + 1 < split;  // the next level's first sweep
-    // four lanes to a coarse cell, one per fine cell of its aggregate
-    for (int q = lp.start; q < ((4 * C.n + 31) & ~31); q += lp.stride) {
-      const int Q = q >> 2, k = C.dplane(Q), r = Q - k * C.dplane.d, J = C.dnx(r), I = r - J * C.nx;
-      const int i = 2 * I + (q & 1), j = 2 * J + ((q >> 1) & 1), f = k * plane + j * L.nx + i;
-      double res = 0.0;
-      if (Q < C.n && i < L.nx && j < L.ny) res = rhs[f] - apply(L, xa, f);
-      const double r1 = __shfl_down_sync(0xffffffffu, res, 1), r2 = __shfl_down_sync(0xffffffffu, res, 2),
-                   r3 = __shfl_down_sync(0xffffffffu, res, 3);
-      if ((q & 3) == 0 && Q < C.n) {
-        const double acc = 0.0 + res + r1 + r2 + r3;  // cells beyond the edge count 0
+    // One thread to a coarse cell, or, where that leaves threads idle, four
+    // lanes, one per fine cell (an 18 k-cell level: 4.4 -> 1.8 us; 4.5 M cells:
+    // 72 us by lanes, 64 by threads).
+    if (C.n >= lp.stride) {
+      for (int Q = lp.start; Q < C.n; Q += lp.stride) {
+        const int k = C.dplane(Q), r = Q - k * C.dplane.d, J = C.dnx(r), I = r - J * C.nx;
+        const int f = k * plane + 2 * J * L.nx + 2 * I;
+        const bool e = 2 * I + 1 < L.nx, nn = 2 * J + 1 < L.ny;
+        double acc = 0.0 + (rhs[f] - apply(L, xa, f));
+        if (e) acc += rhs[f + 1] - apply(L, xa, f + 1);
+        if (nn) acc += rhs[f + L.nx] - apply(L, xa, f + L.nx);
+        if (e && nn) acc += rhs[f + L.nx + 1] - apply(L, xa, f + L.nx + 1);
         C.b[Q] = acc;
         if (first) C.x0[Q] = cps::div_rn(w * acc, C.c[kD][Q]);
+      }
+    } else {
+      for (int q = lp.start; q < ((4 * C.n + 31) & ~31); q += lp.stride) {
+        const int Q = q >> 2, k = C.dplane(Q), r = Q - k * C.dplane.d, J = C.dnx(r), I = r - J * C.nx;
+        const int i = 2 * I + (q & 1), j = 2 * J + ((q >> 1) & 1), f = k * plane + j * L.nx + i;
+        double res = 0.0;
+        if (Q < C.n && i < L.nx && j < L.ny) res = rhs[f] - apply(L, xa, f);
+        const double r1 = __shfl_down_sync(0xffffffffu, res, 1), r2 = __shfl_down_sync(0xffffffffu, res, 2),
+                     r3 = __shfl_down_sync(0xffffffffu, res, 3);
+        if ((q & 3) == 0 && Q < C.n) {
+          const double acc = 0.0 + res + r1 + r2 + r3;  // cells beyond the edge count 0
+          C.b[Q] = acc;
+          if (first) C.x0[Q] = cps::div_rn(w * acc, C.c[kD][Q]);
+        }
       }
     }
     if (!g.sync()) { ok = false; return a0; }
