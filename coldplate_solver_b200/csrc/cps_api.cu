@@ -5,14 +5,14 @@
 // p, p', u*, v*, dE, dN, alpha, gamma) come first, each (M+1) rows x P
 // doubles, P = round_up(N+1, 32); then the 25 inner-solve planes in the
 // context's storage type (double for CPS_FP64, float for CPS_MIXED); then the
-// grid barrier, flags, reduction ring and history buffer.  The fields stay
-// resident between calls; per outer iteration only the 8 diagnostics travel
-// to the host (batched per call).
+// grid barrier, flags, history buffer (one copy to the host per launch takes
+// the two) and reduction ring.  The fields stay resident between calls; per
+// outer iteration only the 8 diagnostics travel to the host.
 //
 // Launch, one design: the outer iterations run in one persistent kernel
-// launched cooperatively (all CTAs co-resident), synchronised by a software
-// grid barrier whose waits are bounded (2 s) and report CPS_ERR_TIMEOUT
-// instead of hanging.
+// launched cooperatively (all CTAs co-resident; in clusters of 16 where one of
+// them runs the PCG), synchronised by a software grid barrier whose waits are
+// bounded (2 s) and report CPS_ERR_TIMEOUT instead of hanging.
 //
 // Launch, many designs (cps_batch_solve): one thread-block cluster per design
 // at a time; clusters take designs from a device work queue, synchronise with
@@ -27,6 +27,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <exception>
 #include <mutex>
 #include <new>
 #include <numeric>
@@ -312,10 +313,14 @@ bool download_planes(cps_ctx* c, const PlaneOut* planes, int n, int layout) {
   const size_t slot = stage / ((size_t)threads * depth);
   struct Chunk { int plane, row, rows; };
   std::vector<Chunk> chunks;
-  for (int k = 0; k < n; ++k) {
-    if (!planes[k].dst) continue;
-    const int per = (int)(slot / planes[k].cols);
-    for (int r = 0; r < planes[k].rows; r += per) chunks.push_back({k, r, std::min(per, planes[k].rows - r)});
+  try {
+    for (int k = 0; k < n; ++k) {
+      if (!planes[k].dst) continue;
+      const int per = (int)(slot / planes[k].cols);
+      for (int r = 0; r < planes[k].rows; r += per) chunks.push_back({k, r, std::min(per, planes[k].rows - r)});
+    }
+  } catch (const std::exception&) {
+    return cuda_ok(c, cudaErrorMemoryAllocation, "download");
   }
   std::atomic<int> failed{cudaSuccess};
   auto worker = [&](int t) {

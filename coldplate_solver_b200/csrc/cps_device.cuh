@@ -55,9 +55,10 @@
 // u*, v* and z0 once per tile over the halo instead of once per neighbour.
 // The Jacobi sweeps of B read global memory directly (a TMA-staged form is
 // kept behind CPS_STAGE_SWEEPS=1; it measured no faster); P1 and P2 keep their
-// state in registers or shared memory when it fits, else read global memory
-// directly.  Per-point expressions and per-thread summation order are the
-// same either way, so the results do not depend on staging.
+// state on chip as far as it fits (a cluster's shared memory, registers and
+// shared memory, p alone), else read global memory directly.  Per-point
+// expressions and per-thread summation order are the same either way, so the
+// results do not depend on staging.
 #pragma once
 #include <cuda_runtime.h>
 #include <cooperative_groups.h>
@@ -2019,8 +2020,8 @@ inline __host__ __device__ int pcg_form(int M, int N, int nblk) {
 // p = z + beta p on the fly for the 5-point stencil and Ap; phase P2 updates
 // x, r, z.  rz0 = r0.z0 and pAp0 = p0.A p0 come from phase C.  From iteration
 // 1 on the CTAs hold their tiles on chip (pcg_tiles), or p of them (pcg_stream),
-// when they fit, else read global memory (pcg_global).  Returns the reference's iteration count, or -1
-// if a wait failed.
+// when they fit, else read global memory (pcg_global).  Returns the
+// reference's iteration count, or -1 if a wait failed.
 // ---------------------------------------------------------------------------
 template <typename T, int Carry, class Group>
 __device__ __forceinline__ int pcg_two_reductions(const DesignView& d, Group& g, double* smem, char* tbuf, double rz0,

@@ -412,7 +412,8 @@ __device__ __forceinline__ void local_vcycle(const View& tv, const double* __res
 // B200, ms per solve with five phases per level, index divisions in the
 // stencil and the small levels out of global memory -> now: 100 x 40 x 9
 // 2.9 -> 1.9, 250 x 125 x 9 8.7 -> 5.4, 500 x 240 x 9 23.2 -> 16.0,
-// 1000 x 500 x 9 95 -> 80.
+// 1000 x 500 x 9 95 -> 80 (75.7 with the restriction rule and the vector
+// updates below).
 // ---------------------------------------------------------------------------
 __device__ double* vcycle(const View& tv, cps::GridGroup& g, const double* rhs0, double* a0, double* a1, double* sm,
                           bool& ok) {
