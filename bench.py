@@ -616,7 +616,7 @@ THERMAL_METRIC = "converged thermal solves/s (relative residual 1e-6)"
 # DRAM bytes (read + write) per launch of the thermal solve on the full
 # 1000 x 500 x 9 workload (63 BiCGStab iterations), from a one-pass ncu launch
 # list; profiles/cpt_solve_kernel_thermal_density_fp64.txt has the command.
-THERMAL_TRAFFIC = 3.058e11
+THERMAL_TRAFFIC = 3.091e11
 
 
 def thermal_bytes_per_iteration(n_levels_cells) -> float:
@@ -1047,9 +1047,9 @@ def run_many(args) -> None:
 # workload (`bench.py --steps 2 --warmup 3 --no-cpu-baseline`, 14 launches,
 # FP64); profiles/cps_grid_kernel_network_500x250_fp64.txt has the command.
 # Density 1000 x 500: two launches of the full workload (the first, early launch
-# of a solve and the next, late one), 596.4 and 595.9 GB
+# of a solve and the next, late one), 578.5 and 575.7 GB
 # (profiles/cps_grid_kernel_density_1000x500_fp64.txt has the command).
-MEASURED_TRAFFIC = {("network", "fp64"): 1.249e9, ("density", "fp64"): 5.962e11}
+MEASURED_TRAFFIC = {("network", "fp64"): 1.249e9, ("density", "fp64"): 5.771e11}
 
 # Outer iterations of a converged FP64 solve of each workload (1e-6 outer
 # residual): straight and network by the bit-exact FP64 oracle (the
