@@ -116,6 +116,7 @@ enum TmaMap : int {
 // design needs.
 enum Carries : int { kFew = 1, kMany = 2, kLarge = 4, kForms = 7, kOptions = 8, kAll = 15, kCluster = 16 };
 
+// A design that diverged runs its step to the end; a timeout replaces either.
 enum DeviceStatus : int { kStatusOk = 0, kStatusTimeout = 1, kStatusDiverged = 2 };
 
 // Inner-solve arrays of one design in storage type T.
@@ -556,6 +557,8 @@ struct GridGroup {
   }
 
   // Thread 0 only: arrive at barrier number `epoch` and wait for the others.
+  // Only a wait that ran out of time ends the others: a step that diverged is
+  // finished by every CTA, so that its fields do not depend on who polled when.
   __device__ int arrive_and_wait() {
     const unsigned long long target = epoch * nblk;
     const unsigned long long old = atom_add_acq_rel_u64(&bar->count, 1ull);
@@ -564,9 +567,9 @@ struct GridGroup {
     unsigned spins = 0;
     while (ld_acquire_u64(&bar->count) < target) {
       if ((++spins & 255u) == 0) {
-        if (*(volatile int*)status != kStatusOk) return 0;
+        if (*(volatile int*)status == kStatusTimeout) return 0;
         if (globaltimer_ns() - t0 > kBarrierTimeoutNs) {
-          atomicCAS(status, kStatusOk, kStatusTimeout);
+          atomicExch(status, kStatusTimeout);
           return 0;
         }
       }
@@ -935,7 +938,7 @@ __device__ __forceinline__ bool for_each_tile(const DesignView& d, Group& g, cha
     if (__syncthreads_or(late)) {
       // a tile copy did not land: record it, wait (bounded) for this tile's
       // and the later tiles' copies still in flight, and stop
-      if (threadIdx.x == 0 && g.status) atomicCAS(g.status, kStatusOk, kStatusTimeout);
+      if (threadIdx.x == 0 && g.status) atomicExch(g.status, kStatusTimeout);
       for (int q = 0; q < kStageDepth; ++q)
         if (t + q * (int)nblk < nt) {
           const int b = (k + q) % kStageDepth;
@@ -1853,8 +1856,31 @@ __device__ __forceinline__ void fold_tiles(const double* p0, const double* p1, i
   s0 = a;
   s1 = b;
 }
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_arrive() {
+  __syncwarp();  // .aligned: by all lanes together
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
+// The cluster's CTAs store into one another's shared memory, so none of them
+// leaves the kernel while another may still do so.  A CTA whose wait failed
+// (anywhere in the outer iteration) tells the others here and arrives at the
+// cluster barrier; they meet it there, at the end of their own run or in
+// pcg_cluster, whose first barrier ends the PCG when the word is set
+// (kLeft).  Every CTA of the cluster calls enter before any of them stores
+// to another and leave unless it got kLeft.
+constexpr int kLeft = -2;  // outer_iteration: the cluster has left together
+__shared__ int s_cluster_leave;
+__device__ __forceinline__ void cluster_enter() {
+  if (threadIdx.x == 0) s_cluster_leave = 0;
+  cluster_arrive();
+  cluster_wait();
+}
+__device__ __forceinline__ void cluster_leave(bool failed) {
+  if (failed && threadIdx.x < kClusterCtas) *cg::this_cluster().map_shared_rank(&s_cluster_leave, threadIdx.x) = 1;
+  cluster_arrive();
+  cluster_wait();
+}
 
 template <typename T>
 __device__ __forceinline__ int pcg_cluster(const DesignView& d, int rank, char* tbuf, double alpha0, double rz,
@@ -1960,6 +1986,7 @@ __device__ __forceinline__ int pcg_cluster(const DesignView& d, int rank, char* 
     }
     cluster_arrive();
     cluster_wait();
+    if (it == 1 && *(volatile int*)&s_cluster_leave) return kLeft;
     double pAp, unused;
     fold_tiles(S.part1, S.part1, tiles, pAp, unused);
     if (fabs(pAp) < 1e-20) break;
@@ -2043,6 +2070,7 @@ __device__ __forceinline__ int pcg_two_reductions(const DesignView& d, Group& g,
   const double rz = s2[1], beta = div_uniform(rz, rz0);
   if constexpr (Carry == kCluster) {
     const int its = g.rank < (unsigned)kClusterCtas ? pcg_cluster<T>(d, (int)g.rank, tbuf, alpha, rz, beta) : 0;
+    if (its == kLeft) return kLeft;
     return g.sync() ? its : -1;  // the count is CTA 0's to report
   }
   if constexpr ((Carry & kFew) != 0)
@@ -2696,7 +2724,7 @@ __device__ __forceinline__ bool tile_buffer_fits(const char* dyn, size_t bytes, 
 // pseudo-transient term and the controllers out.  Returns 0 to continue with another outer
 // iteration, 1 when this one is the last (iteration budget, convergence, the
 // pressure-drop gate, or a non-finite residual), -1 when the group must stop
-// because a device-side wait failed.
+// because a device-side wait failed (kLeft: and the PCG's cluster has left).
 // ---------------------------------------------------------------------------
 template <typename T, class Group, bool Monitor = false, bool Pseudo = true, int Carry = kAll>
 __device__ int outer_iteration(const DesignView& d, Group& g, double* smem, char* tbuf, double* out,
@@ -2874,7 +2902,7 @@ __device__ int outer_iteration(const DesignView& d, Group& g, double* smem, char
     if (threadIdx.x == 0) out[5] = its;
   } else {
     const int its = pcg_two_reductions<T, Carry>(d, g, smem, tbuf, rc[5], rc[6]);
-    if (its < 0) return -1;
+    if (its < 0) return its;
     if (threadIdx.x == 0) out[5] = its;
   }
   // ---- D: pressure and velocity correction ----
