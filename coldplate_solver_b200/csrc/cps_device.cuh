@@ -477,6 +477,7 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const TensorMap* map, int
       : "memory");
 }
 __device__ __forceinline__ void fence_proxy_async_shared() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+__device__ __forceinline__ void fence_proxy_async_global() { asm volatile("fence.proxy.async.global;" ::: "memory"); }
 
 // The CTA's stage-buffer mbarriers and the parity of each one's next phase
 // (one byte per buffer: thread 0 flips buffer b's byte while others may read
@@ -913,9 +914,12 @@ __device__ __forceinline__ bool for_each_tile(const DesignView& d, Group& g, cha
     }
   };
   if (tm) {
-    // earlier generic-proxy accesses to the buffers come before the copies
+    // earlier generic-proxy accesses to the buffers come before the copies, and
+    // so do the planes' values that other CTAs stored before the last barrier
+    // (thread 0 acquired them there and issues the copies)
     fence_proxy_async_shared();
     __syncthreads();
+    if (threadIdx.x == 0) fence_proxy_async_global();
   }
 #pragma unroll
   for (int k = 0; k < kStageDepth - 1; ++k) {
