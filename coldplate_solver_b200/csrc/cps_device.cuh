@@ -256,23 +256,36 @@ __device__ __forceinline__ double mind(double a, double b) { return (b < a) ? b 
 __device__ __forceinline__ double clampd(double v, double lo, double hi) { return (v < lo) ? lo : (hi < v) ? hi : v; }
 
 // ---------------------------------------------------------------------------
-// Correctly rounded division without a branch.  The quotient is corrected once
-// from its exact remainder (Markstein, IBM J. Res. Dev. 34, 1990): with y =
-// 1/b rounded to nearest, q = a y and r = a - b q (exact under fma), q + r y
-// is a/b rounded to nearest, the value `/` returns.  y comes from two Newton
-// steps on the hardware's reciprocal approximation and is shared by divisions
-// with a divisor in common.
+// Correctly rounded division without a branch, for positive divisors.  The
+// quotient is corrected once from its exact remainder (Markstein, IBM J. Res.
+// Dev. 34, 1990): with y = 1/b rounded to nearest, q = a y and r = a - b q
+// (exact under fma), q + r y is a/b rounded to nearest, the value `/` returns.
+// y is shared by divisions with a divisor in common.
+//
+// y takes two Newton steps from the hardware's reciprocal approximation, whose
+// relative error e < 2^-18.5 they leave as e^4: y may then be the wrong one of
+// 1/b's two neighbours where 1/b is that close to their middle.  The quotient
+// suffers only where b's significand is so close to 2 that the remainder's
+// rounding error, b^2 (1 + 2^54 e^4) in units of 2^106 for 53-bit integers b,
+// reaches 1: b = 2^53 - k with k <= 2^106 e^4, so k < 2^32.  There the
+// approximation is the power of two itself and e = 2^-53 k, for which no k
+// does, except k = 1, all ones, Markstein's exception: 1/b rounds to the power
+// of two's upper neighbour, and the step's result to the power.  (Both
+// properties of the approximation are tested over all 2^20 significands that
+// it tells apart.)
 //
 // Why: `/` guards its operands with a branch, so consecutive divisions of a
 // thread do not overlap, and a zero numerator (solid cells, fields not yet
 // reached from the zero state) takes its out-of-line path.  Measured on B200,
 // divisions per SM and clock at 512 threads: `/` 3.5, `/` with zero numerators
-// 0.9, this 6.0 either way; per division of one warp 130, 434 and 35 clocks.
+// 0.9, this 4.7 either way; per division of one warp 130, 434 and 45 clocks.
 //
-// Range: y must be normal (2^-1000 <= |b| <= 2^1000 here: the divisors are
-// relaxed momentum diagonals >= 1e-10 and pressure diagonals >= 1e-20).  For
-// quotients below 2^-960 the remainder may underflow and the last bit is not
-// guaranteed; an infinite numerator or an overflowing quotient gives q.
+// Range: 2^-1000 <= b <= 2^1000 (the divisors are relaxed momentum diagonals
+// >= 1e-10, pressure diagonals >= 1e-20, the heat solve's diagonals >= 1e-12
+// and its coarsest column's pivots).  For numerators below 2^-960 the
+// remainder may underflow, and a quotient below 2^-1022 is rounded twice: the
+// last bit is not guaranteed there.  A zero numerator keeps its sign; an
+// infinite numerator or an overflowing quotient gives q.
 // ---------------------------------------------------------------------------
 // c ? a : b with both evaluated: no branch for the compiler to put around a
 // division, so that a thread's divisions overlap.
@@ -283,15 +296,25 @@ __device__ __forceinline__ double select(bool c, double a, double b) {
 }
 // One Newton step of y towards 1/b.
 __device__ __forceinline__ double recip_step(double b, double y) { return __fma_rn(y, __fma_rn(-b, y, 1.0), y); }
-__device__ __forceinline__ double recip(double b) {
+// The last step, with the exception.
+__device__ __forceinline__ double recip_last(double b, double y) {
+  y = recip_step(b, y);
+  const bool ones = ((__double2hiint(b) | ~0xfffff) & __double2loint(b)) == -1;
+  return __hiloint2double(__double2hiint(y), ones ? 1 : __double2loint(y));
+}
+// 1/b from y within a few units of its last place.
+__device__ __forceinline__ double recip_from(double b, double y) { return recip_last(b, recip_step(b, y)); }
+__device__ __forceinline__ double recip_approx(double b) {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
-  return recip_step(b, recip_step(b, y));
+  return y;
 }
+__device__ __forceinline__ double recip(double b) { return recip_from(b, recip_approx(b)); }
 // a / b with y = recip(b).
 __device__ __forceinline__ double div_rn(double a, double b, double y) {
   const double q = a * y;
-  const double v = __fma_rn(__fma_rn(-b, q, a), y, q);
+  // -r, so that a zero numerator's remainder adds a zero of either sign to q as it is
+  const double v = __fma_rn(-__fma_rn(b, q, -a), y, q);
   return select((__double2hiint(v) & 0x7ff00000) == 0x7ff00000, q, v);
 }
 __device__ __forceinline__ double div_rn(double a, double b) { return div_rn(a, b, recip(b)); }
@@ -1078,7 +1101,7 @@ __device__ __forceinline__ MomRow momentum_row(const DesignView& d, const Layout
   if (d.conv == 1) Sp += sou_correction<IsU>(d, X, i, j, Fe, Fw, Fn, Fs);
   const double rAP0 = recip(aP0);
   dOut = div_rn(IsU ? d.hy : d.hx, aP0, rAP0);
-  m.rAP = recip_step(m.aP, d.uvAlpha * rAP0);
+  m.rAP = recip_from(m.aP, d.uvAlpha * rAP0);
   const int iHi = IsU ? M - 1 : M - 2, jHi = IsU ? N - 2 : N - 1;
   m.hasE = j + 1 <= jHi;
   m.hasW = j - 1 >= 1;
