@@ -1672,7 +1672,9 @@ __device__ __forceinline__ int pcg_tiles(const DesignView& d, Group& g, double* 
 // this replaces there, an iteration moves 88 instead of 120 bytes per unknown
 // and touches seven vectors instead of nine: 117 MB instead of 151 MB on the
 // 2048 x 1024 design (28 tiles per CTA), which the 126 MB L2 holds; there an
-// iteration takes 41 instead of 75 us (FP64).
+// iteration takes 41 instead of 75 us (FP64).  Column 0 of cx and row 0 of cy,
+// which no phase writes, are read and count for nothing: the caller keeps them
+// finite (contexts and cps_solve_noalloc clear them).
 // ---------------------------------------------------------------------------
 template <typename T>
 struct PcgStreamCount {

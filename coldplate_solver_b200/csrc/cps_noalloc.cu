@@ -186,6 +186,13 @@ extern "C" cps_status cps_solve_noalloc(const cps_desc* desc, int pitch, const d
   for (double* out : {pStar, uStar, vStar, dE, dN})
     if (e == cudaSuccess) e = cudaMemsetAsync(out, 0, rows, st);
   if (e == cudaSuccess) e = cudaMemsetAsync(flags, 0, kFlagsBytes, st);
+  // So do the conductances west of the first column and south of the first row,
+  // which no phase writes and pcg_stream reads: the scratch holds what the last
+  // call, of any shape and outcome, left there.
+  if (cps::pcg_form<double>(d.M, d.N, grid) == cps::kLarge) {
+    if (e == cudaSuccess) e = cudaMemset2DAsync(w.f64.cx, (size_t)pitch * sizeof(double), 0, sizeof(double), d.M + 1, st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(w.f64.cy, 0, (size_t)pitch * sizeof(double), st);
+  }
   if (e != cudaSuccess) return fail(CPS_ERR_CUDA, std::string("memset: ") + cudaGetErrorString(e));
   cps::RunControl rc{max_outer, eps > 0.0 ? 1 : 0, eps, hist, done, status};
   void* args[] = {&w, &rc, &bar, &ring};
