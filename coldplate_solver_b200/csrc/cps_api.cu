@@ -97,6 +97,8 @@ CPS_GRID_KERNELS(extern, double)
 CPS_GRID_KERNELS(extern, float)
 CPS_GRID_OPTION_KERNELS(extern, double)
 CPS_GRID_OPTION_KERNELS(extern, float)
+CPS_GRID_MONITOR_KERNELS(extern, double)
+CPS_GRID_MONITOR_KERNELS(extern, float)
 CPS_BATCH_KERNELS(extern, double)
 CPS_BATCH_KERNELS(extern, float)
 CPS_BATCH_OPTION_KERNELS(extern, double)
@@ -393,9 +395,13 @@ void set_step_inputs(cps_ctx* c, double Uin) {
 }
 
 // The single-design kernels of a storage type, each with the dynamic shared
-// memory it needs: one per PCG form on the default path, then the ones that
-// carry every option, without and with the monitor, then the one whose PCG
-// runs on one cluster (8 x 32 tiles only).
+// memory it needs: one per PCG form on the default path, with every option,
+// and with the monitor and every option, then the one whose PCG runs on one
+// cluster (8 x 32 tiles only).  One form each: with all of them in one kernel
+// (136 bytes of spills; 0, 60 and 0 for the three forms) a late outer
+// iteration took, us in FP64: monitored 39.1 instead of 35.9 (256 x 128), 81.0
+// instead of 76.1 (512 x 256) and 132.3 instead of 128.6 (1000 x 500); with
+// the pseudo-transient term 146.5 instead of 141.5 (500 x 250 network).
 struct GridKernel {
   const void* fn;
   size_t smem;
@@ -404,15 +410,20 @@ template <typename T, bool Monitor, bool Pseudo, int Carry>
 GridKernel grid_kernel() {
   return {(const void*)cps_grid_kernel<T, Monitor, Pseudo, Carry>, cps::kernel_smem_bytes<T, Carry, Monitor>()};
 }
-enum GridKernels : int { kGridFew, kGridMany, kGridLarge, kGridOptions, kGridMonitor, kGridKernels, kGridCluster = kGridKernels };
+enum GridForm : int { kGridFew, kGridMany, kGridLarge, kGridForms };
+enum GridKernels : int { kGridPlain = 0, kGridOptions = kGridForms, kGridMonitor = 2 * kGridForms, kGridKernels = 3 * kGridForms, kGridCluster = kGridKernels };
 template <typename T>
 GridKernel grid_kernel(int k) {
   switch (k) {
-    case kGridFew: return grid_kernel<T, false, false, cps::kFew>();
-    case kGridMany: return grid_kernel<T, false, false, cps::kMany>();
-    case kGridLarge: return grid_kernel<T, false, false, cps::kLarge>();
-    case kGridOptions: return grid_kernel<T, false, true, cps::kAll>();
-    case kGridMonitor: return grid_kernel<T, true, true, cps::kAll>();
+    case kGridPlain + kGridFew: return grid_kernel<T, false, false, cps::kFew>();
+    case kGridPlain + kGridMany: return grid_kernel<T, false, false, cps::kMany>();
+    case kGridPlain + kGridLarge: return grid_kernel<T, false, false, cps::kLarge>();
+    case kGridOptions + kGridFew: return grid_kernel<T, false, true, cps::kFew | cps::kOptions>();
+    case kGridOptions + kGridMany: return grid_kernel<T, false, true, cps::kMany | cps::kOptions>();
+    case kGridOptions + kGridLarge: return grid_kernel<T, false, true, cps::kLarge | cps::kOptions>();
+    case kGridMonitor + kGridFew: return grid_kernel<T, true, true, cps::kFew | cps::kOptions>();
+    case kGridMonitor + kGridMany: return grid_kernel<T, true, true, cps::kMany | cps::kOptions>();
+    case kGridMonitor + kGridLarge: return grid_kernel<T, true, true, cps::kLarge | cps::kOptions>();
 #if CPS_TILE_J == 32
     case kGridCluster: return grid_kernel<T, false, false, cps::kCluster>();
 #endif
@@ -429,12 +440,12 @@ bool has_options(const cps::DesignView& v) {
 }
 
 int grid_kernel_for(const cps_ctx* c) {
-  if (c->view.dpMonitor) return kGridMonitor;
-  if (has_options(c->view)) return kGridOptions;
-  if (c->cluster) return kGridCluster;
+  const bool monitor = c->view.dpMonitor != 0, options = has_options(c->view);
+  if (c->cluster && !monitor && !options) return kGridCluster;
   const int form = c->precision == CPS_MIXED ? cps::pcg_form<float>(c->M, c->N, c->grid)
                                              : cps::pcg_form<double>(c->M, c->N, c->grid);
-  return form == cps::kFew ? kGridFew : form == cps::kMany ? kGridMany : kGridLarge;
+  return (monitor ? kGridMonitor : options ? kGridOptions : kGridPlain) +
+         (form == cps::kFew ? kGridFew : form == cps::kMany ? kGridMany : kGridLarge);
 }
 
 // Dynamic shared memory of the persistent kernels (tile staging buffers).

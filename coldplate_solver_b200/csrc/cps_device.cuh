@@ -2089,7 +2089,7 @@ __device__ __forceinline__ int pcg_two_reductions(const DesignView& d, Group& g,
   double s2[2] = {0.0, 0.0};
   bool ok;
   if constexpr (Carry == kCluster) ok = pcg_first<T, false, 1>(d, g, smem, alpha, s2);
-  else if constexpr (Carry == kFew) ok = pcg_first<T, false, kFewTiles>(d, g, smem, alpha, s2);
+  else if constexpr ((Carry & kForms) == kFew) ok = pcg_first<T, false, kFewTiles>(d, g, smem, alpha, s2);
   else if constexpr ((Carry & kLarge) == 0) ok = pcg_first<T, false, 4>(d, g, smem, alpha, s2);
   else if constexpr ((Carry & kForms) == kLarge) ok = pcg_first<T, true, 4>(d, g, smem, alpha, s2);
   else ok = form == kLarge ? pcg_first<T, true, 4>(d, g, smem, alpha, s2) : pcg_first<T, false, 4>(d, g, smem, alpha, s2);

@@ -232,9 +232,12 @@ __global__ void __launch_bounds__(cps::kThreads, CPS_MIN_BLOCKS) cps_wave_kernel
 #else
 #define CPS_GRID_CLUSTER_KERNELS(PRE, T)
 #endif
-#define CPS_GRID_OPTION_KERNELS(PRE, T)                                                                             \
-  CPS_GRID_KERNEL(PRE, T, false, true, cps::kAll)                                                                   \
-  CPS_GRID_KERNEL(PRE, T, true, true, cps::kAll)
+#define CPS_GRID_OPTION_KERNELS_OF(PRE, T, MONITOR)                                                                 \
+  CPS_GRID_KERNEL(PRE, T, MONITOR, true, cps::kFew | cps::kOptions)                                                 \
+  CPS_GRID_KERNEL(PRE, T, MONITOR, true, cps::kMany | cps::kOptions)                                                \
+  CPS_GRID_KERNEL(PRE, T, MONITOR, true, cps::kLarge | cps::kOptions)
+#define CPS_GRID_OPTION_KERNELS(PRE, T) CPS_GRID_OPTION_KERNELS_OF(PRE, T, false)
+#define CPS_GRID_MONITOR_KERNELS(PRE, T) CPS_GRID_OPTION_KERNELS_OF(PRE, T, true)
 #define CPS_BATCH_KERNELS_OF(PRE, T, OPTIONS, CARRY)                                                                \
   PRE template __global__ void cps_cluster_kernel<T, OPTIONS, CARRY>(const cps::BatchItem*, const int*, int, int*,  \
                                                                      cps::BatchResult*);                            \
