@@ -87,6 +87,7 @@ struct cps_ctx {
   int iter = 0;              // outer-loop iteration index of the next iteration (monitor and gate)
   int grid = 0;
   bool cluster = false;      // the PCG may run on one thread-block cluster (cps::kCluster)
+  unsigned ready = 0;        // bit k: grid kernel k is loaded and may use its dynamic shared memory
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   double kernel_ms = 0.0;
   long long launches = 0, outer_done = 0;
@@ -463,6 +464,24 @@ void to_step_out(const double* h, cps_step_out* o) {
   o->pIters = (int)h[5]; o->uSweeps = (int)h[6]; o->vSweeps = (int)h[7];
 }
 
+// The shared memory that every grid kernel is allowed, whichever of them needs
+// it: one value, so that contexts on several threads never lower each other's.
+size_t grid_smem(int precision) {
+  size_t most = 0;
+  for (int k = 0; k < kGridKernels; ++k) most = std::max(most, grid_kernel_of(precision, k).smem);
+  return most;
+}
+
+// Before a context's first launch of a kernel (which loads it); the cluster
+// form's is use_cluster's to prepare.
+bool ready_grid(cps_ctx* c) {
+  const int k = grid_kernel_for(c);
+  if (k == kGridCluster || (c->ready >> k & 1u)) return true;
+  if (!allow_smem(c, grid_kernel_of(c->precision, k).fn, grid_smem(c->precision))) return false;
+  c->ready |= 1u << k;
+  return true;
+}
+
 // The persistent kernel's launch: cooperative (all CTAs co-resident), in
 // clusters where its PCG runs on one.
 cudaError_t launch_grid(const cps_ctx* c, void** args) {
@@ -538,7 +557,7 @@ cps_status run(cps_ctx* c, int n_outer, int stop_on_conv, double eps, cps_step_o
     if (!cuda_ok(c, cudaMemsetAsync(c->bar, 0, kFlagsAt + 4 * sizeof(int), c->stream), "memset"))
       return CPS_ERR_CUDA;
     void* args[] = {&c->view, &rc, &c->bar, &c->red};
-    if (!cuda_ok(c, cudaEventRecord(c->ev0, c->stream), "event")) return CPS_ERR_CUDA;
+    if (!ready_grid(c) || !cuda_ok(c, cudaEventRecord(c->ev0, c->stream), "event")) return CPS_ERR_CUDA;
     if (!cuda_ok(c, launch_grid(c, args), "cooperative launch")) return CPS_ERR_CUDA;
     if (!cuda_ok(c, cudaEventRecord(c->ev1, c->stream), "event")) return CPS_ERR_CUDA;
     if (monitor && dp_history &&
@@ -823,17 +842,19 @@ cps_status cps_create(const cps_desc* d, cps_ctx** out) {
       !upload_plane(c, v.gamma, d->gamma, d->M, d->N, d->layout))
     return bail(CPS_ERR_CUDA);
 
-  // Persistent grid: co-resident CTAs, at most one per tile of the design.
+  // Persistent grid: co-resident CTAs, at most one per tile of the design.  The
+  // kernels are interchangeable within a design, so the grid is what all of
+  // them allow: their launch bounds allow CPS_MIN_BLOCKS CTAs per SM, and the
+  // shared memory of the largest is asked of one of them.  (Asking every kernel
+  // loads every kernel: the first context of a process took 9.3 instead of
+  // 7.5 ms, later ones 2.9 instead of 2.6 ms.)
   int per_sm = 0, sms = 0;
-  for (int k = 0; k < kGridKernels; ++k) {
-    // the kernels are interchangeable within a design, so the grid is what all of them allow
-    const GridKernel kern = grid_kernel_of(d->precision, k);
-    int n = 0;
-    if (!allow_smem(c, kern.fn, kern.smem) ||
-        !cuda_ok(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern.fn, cps::kThreads, kern.smem), "occupancy"))
-      return bail(CPS_ERR_CUDA);
-    per_sm = k == 0 ? n : std::min(per_sm, n);
-  }
+  const size_t most = grid_smem(d->precision);
+  const GridKernel any = grid_kernel_of(d->precision, kGridPlain + kGridFew);
+  if (!allow_smem(c, any.fn, most) ||
+      !cuda_ok(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, any.fn, cps::kThreads, most), "occupancy"))
+    return bail(CPS_ERR_CUDA);
+  per_sm = std::min(per_sm, CPS_MIN_BLOCKS);
   if (!cuda_ok(c, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, d->device), "attribute"))
     return bail(CPS_ERR_CUDA);
   if (per_sm < 1) return bail(fail(c, CPS_ERR_CUDA, "persistent kernel does not fit on an SM"));
@@ -847,6 +868,7 @@ cps_status cps_create(const cps_desc* d, cps_ctx** out) {
   grid = std::max(1, std::min(grid, tiles));
   c->grid = grid;
   c->cluster = use_cluster(c, d);
+  if (!ready_grid(c)) return bail(CPS_ERR_CUDA);
   *out = c;
   return CPS_OK;
 }
