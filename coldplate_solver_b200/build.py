@@ -36,7 +36,7 @@ SOURCES = [os.path.join(PKG_DIR, "csrc", f) for f in (
     "cps_grid_f64.cu", "cps_grid_f32.cu", "cps_grid_opt_f64.cu", "cps_grid_opt_f32.cu", "cps_grid_mon_f64.cu",
     "cps_grid_mon_f32.cu", "cps_batch_f64.cu", "cps_batch_f32.cu", "cps_batch_opt_f64.cu", "cps_batch_opt_f32.cu",
     "cps_api.cu", "cps_noalloc.cu", "cps_thermal.cu", "cps_io.cpp", "cps_thermal_io.cpp")]
-HEADERS = [os.path.join(PKG_DIR, "csrc", f) for f in os.listdir(os.path.join(PKG_DIR, "csrc")) if f.endswith(".cuh")]
+HEADERS = [os.path.join(PKG_DIR, "csrc", f) for f in os.listdir(os.path.join(PKG_DIR, "csrc")) if f.endswith((".cuh", ".h"))]
 HEADERS.append(os.path.join(REPO_DIR, "include", "cps.h"))
 HEADERS.append(os.path.join(REPO_DIR, "include", "cps_thermal.h"))
 

@@ -31,6 +31,7 @@ CPS_ERR_ARG, CPS_ERR_OOM, CPS_ERR_CUDA, CPS_ERR_TIMEOUT, CPS_ERR_DIVERGED, CPS_E
 CPS_ROW_MAJOR, CPS_COL_MAJOR = 0, 1
 CPS_FP64, CPS_MIXED = 0, 1
 CPS_PCG_REFERENCE, CPS_PCG_SINGLE_REDUCTION = 0, 1
+CPS_PCG_FORM_NONE, CPS_PCG_FORM_FEW, CPS_PCG_FORM_MANY, CPS_PCG_FORM_LARGE, CPS_PCG_FORM_CLUSTER = range(5)
 
 _STATUS_NAMES = {0: "OK", -1: "CPS_ERR_ARG", -2: "CPS_ERR_OOM", -3: "CPS_ERR_CUDA", -4: "CPS_ERR_TIMEOUT",
                  -5: "CPS_ERR_DIVERGED", -6: "CPS_ERR_STATE"}
@@ -172,6 +173,7 @@ SIGNATURES = {
     "cps_upload_geometry": (ctypes.c_int, [_P, _D, _D, ctypes.c_int]),
     "cps_reset_fields": (ctypes.c_int, [_P]),
     "cps_get_stream": (ctypes.c_int, [_P, ctypes.POINTER(_P)]),
+    "cps_last_pcg_form": (ctypes.c_int, [_P, ctypes.POINTER(ctypes.c_int)]),
     "cps_kernel_timing": (ctypes.c_int, [_P, ctypes.POINTER(ctypes.c_double), ctypes.POINTER(ctypes.c_longlong),
                                          ctypes.POINTER(ctypes.c_longlong), ctypes.c_int]),
     "cps_batch_solve": (ctypes.c_int, [ctypes.POINTER(_P), ctypes.c_int, _D, ctypes.POINTER(CpsBatchOpts),
@@ -365,6 +367,13 @@ class Solver:
         s = _P()
         self._check(self.lib.cps_get_stream(self.ctx, ctypes.byref(s)))
         return int(s.value or 0)
+
+    @property
+    def last_pcg_form(self) -> int:
+        """cps_last_pcg_form: one of the CPS_PCG_FORM_ values."""
+        form = ctypes.c_int(0)
+        self._check(self.lib.cps_last_pcg_form(self.ctx, ctypes.byref(form)))
+        return form.value
 
     def kernel_timing(self, reset: bool = False):
         """(kernel_ms, launches, outer_iterations) since the last reset."""

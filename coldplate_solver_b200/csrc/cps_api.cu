@@ -36,6 +36,7 @@
 #include <vector>
 
 #include "../../include/cps.h"
+#include "cps_host.h"
 #include "cps_kernels.cuh"
 
 namespace {
@@ -87,6 +88,7 @@ struct cps_ctx {
   int iter = 0;              // outer-loop iteration index of the next iteration (monitor and gate)
   int grid = 0;
   bool cluster = false;      // the PCG may run on one thread-block cluster (cps::kCluster)
+  int kernel = -1;           // grid kernel of the last launch
   unsigned ready = 0;        // bit k: grid kernel k is loaded and may use its dynamic shared memory
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   double kernel_ms = 0.0;
@@ -440,9 +442,16 @@ bool has_options(const cps::DesignView& v) {
   return v.pseudo != 0 || v.momExplicit != 0 || v.pcgSingleReduction != 0 || v.stageSweeps != 0;
 }
 
-int grid_kernel_for(const cps_ctx* c) {
+// The kernel of a context's next launch; `alone`: no other launch is in flight
+// on the device.  Beside another launch a design of the cluster form takes the
+// grid form, two CTAs to an SM and the same bits.  B200, channel 200 x 100, 60
+// outer iterations, ms per solve over 1 / 2 / 3 / 6 host threads: always the
+// cluster form 5.4 / 5.3 / 5.3 / 5.3, always the grid form 6.9 / 3.6 / 2.5 /
+// 2.5, this rule 5.4 / 3.5 / 2.4 / 2.4.  (A launch under way keeps its form: a
+// third context may wait for it to end once.)
+int grid_kernel_for(const cps_ctx* c, bool alone) {
   const bool monitor = c->view.dpMonitor != 0, options = has_options(c->view);
-  if (c->cluster && !monitor && !options) return kGridCluster;
+  if (c->cluster && alone && !monitor && !options) return kGridCluster;
   const int form = c->precision == CPS_MIXED ? cps::pcg_form<float>(c->M, c->N, c->grid)
                                              : cps::pcg_form<double>(c->M, c->N, c->grid);
   return (monitor ? kGridMonitor : options ? kGridOptions : kGridPlain) +
@@ -474,8 +483,7 @@ size_t grid_smem(int precision) {
 
 // Before a context's first launch of a kernel (which loads it); the cluster
 // form's is use_cluster's to prepare.
-bool ready_grid(cps_ctx* c) {
-  const int k = grid_kernel_for(c);
+bool ready_grid(cps_ctx* c, int k) {
   if (k == kGridCluster || (c->ready >> k & 1u)) return true;
   if (!allow_smem(c, grid_kernel_of(c->precision, k).fn, grid_smem(c->precision))) return false;
   c->ready |= 1u << k;
@@ -484,8 +492,7 @@ bool ready_grid(cps_ctx* c) {
 
 // The persistent kernel's launch: cooperative (all CTAs co-resident), in
 // clusters where its PCG runs on one.
-cudaError_t launch_grid(const cps_ctx* c, void** args) {
-  const int k = grid_kernel_for(c);
+cudaError_t launch_grid(const cps_ctx* c, int k, void** args) {
   const GridKernel kern = grid_kernel_of(c->precision, k);
   const bool cluster = k == kGridCluster;
   cudaLaunchConfig_t cfg = {};
@@ -557,8 +564,10 @@ cps_status run(cps_ctx* c, int n_outer, int stop_on_conv, double eps, cps_step_o
     if (!cuda_ok(c, cudaMemsetAsync(c->bar, 0, kFlagsAt + 4 * sizeof(int), c->stream), "memset"))
       return CPS_ERR_CUDA;
     void* args[] = {&c->view, &rc, &c->bar, &c->red};
-    if (!ready_grid(c) || !cuda_ok(c, cudaEventRecord(c->ev0, c->stream), "event")) return CPS_ERR_CUDA;
-    if (!cuda_ok(c, launch_grid(c, args), "cooperative launch")) return CPS_ERR_CUDA;
+    const cps::InFlight flight(c->device);
+    c->kernel = grid_kernel_for(c, flight.alone());
+    if (!ready_grid(c, c->kernel) || !cuda_ok(c, cudaEventRecord(c->ev0, c->stream), "event")) return CPS_ERR_CUDA;
+    if (!cuda_ok(c, launch_grid(c, c->kernel, args), "cooperative launch")) return CPS_ERR_CUDA;
     if (!cuda_ok(c, cudaEventRecord(c->ev1, c->stream), "event")) return CPS_ERR_CUDA;
     if (monitor && dp_history &&
         !cuda_ok(c, cudaMemcpyAsync(c->hdplog, c->dplog, sizeof(double) * 4 * chunk, cudaMemcpyDeviceToHost,
@@ -868,7 +877,7 @@ cps_status cps_create(const cps_desc* d, cps_ctx** out) {
   grid = std::max(1, std::min(grid, tiles));
   c->grid = grid;
   c->cluster = use_cluster(c, d);
-  if (!ready_grid(c)) return bail(CPS_ERR_CUDA);
+  if (!ready_grid(c, grid_kernel_for(c, true))) return bail(CPS_ERR_CUDA);
   *out = c;
   return CPS_OK;
 }
@@ -1018,6 +1027,14 @@ cps_status cps_set_pseudo_state(cps_ctx* c, const cps_pseudo_state* state) {
              : CPS_ERR_CUDA;
 }
 
+cps_status cps_last_pcg_form(const cps_ctx* c, int* form) {
+  if (!c || !form) return fail(nullptr, CPS_ERR_ARG, "ctx and form are required");
+  *form = c->kernel < 0                ? CPS_PCG_FORM_NONE
+          : c->kernel == kGridCluster ? CPS_PCG_FORM_CLUSTER
+                                      : CPS_PCG_FORM_FEW + c->kernel % kGridForms;
+  return CPS_OK;
+}
+
 cps_status cps_get_stream(cps_ctx* c, void** stream) {
   if (!c || !stream) return fail(c, CPS_ERR_ARG, "ctx and stream are required");
   *stream = (void*)c->stream;
@@ -1134,6 +1151,7 @@ cps_status cps_batch_solve(cps_ctx* const* ctxs, int n, const double* inletVeloc
   }
   std::lock_guard<std::mutex> lock(g_batch_mutex);
   if (!cuda_ok(c0, cudaSetDevice(c0->device), "cudaSetDevice")) return CPS_ERR_CUDA;
+  const cps::InFlight flight(c0->device);
   std::string err;
   BatchWorkspace* ws = batch_workspace(c0->device, (size_t)n, err);
   if (!ws) return fail(c0, CPS_ERR_OOM, err);

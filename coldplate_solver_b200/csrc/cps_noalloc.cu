@@ -39,6 +39,7 @@
 
 #include "../../include/cps.h"
 #include "cps_device.cuh"
+#include "cps_host.h"
 
 namespace {
 
@@ -194,6 +195,7 @@ extern "C" cps_status cps_solve_noalloc(const cps_desc* desc, int pitch, const d
     if (e == cudaSuccess) e = cudaMemsetAsync(w.f64.cy, 0, (size_t)pitch * sizeof(double), st);
   }
   if (e != cudaSuccess) return fail(CPS_ERR_CUDA, std::string("memset: ") + cudaGetErrorString(e));
+  const cps::InFlight flight(dev);
   cps::RunControl rc{max_outer, eps > 0.0 ? 1 : 0, eps, hist, done, status};
   void* args[] = {&w, &rc, &bar, &ring};
   e = cudaLaunchCooperativeKernel((const void*)cps_noalloc_kernel, dim3(grid), dim3(cps::kThreads), args,

@@ -30,6 +30,7 @@
 
 #include "../../include/cps_thermal.h"
 #include "cps_device.cuh"
+#include "cps_host.h"
 
 namespace cpt {
 
@@ -966,6 +967,7 @@ cps_status solve_launch(cps_thermal* t, int warm, cps_thermal_result* res) {
   cpt::View& tv = t->view;
   if (!tcuda(t, cudaMemsetAsync(tv.out, 0, 32 * sizeof(double), t->stream), "memset")) return CPS_ERR_CUDA;
   double T_in = t->desc.T_inlet;
+  const cps::InFlight flight(t->device);
   void* args[] = {&tv, &T_in, &warm, &t->bar, &t->red, &t->status};
   if (!tcuda(t, cudaEventRecord(t->ev0, t->stream), "event") ||
       !tcuda(t, cudaLaunchCooperativeKernel((const void*)cpt::solve_kernel, dim3(t->grid), dim3(cps::kThreads), args,

@@ -150,6 +150,19 @@ cps_status cps_reset_fields(cps_ctx* ctx);
  * for callers that time or order work against it. */
 cps_status cps_get_stream(cps_ctx* ctx, void** stream);
 
+/* Where the pressure PCG of the context's last single-design launch kept its
+ * state.  The design's size chooses, and whether other launches were in flight
+ * on the device (the cluster form leaves no room beside itself); the results
+ * do not depend on it. */
+enum {
+  CPS_PCG_FORM_NONE = 0,    /* no launch yet */
+  CPS_PCG_FORM_FEW = 1,     /* up to two tiles per CTA, on chip */
+  CPS_PCG_FORM_MANY = 2,    /* more tiles per CTA, on chip */
+  CPS_PCG_FORM_LARGE = 3,   /* the search direction on chip, or nothing */
+  CPS_PCG_FORM_CLUSTER = 4  /* one thread-block cluster's shared memory */
+};
+cps_status cps_last_pcg_form(const cps_ctx* ctx, int* form);
+
 /* Device time of the outer-iteration kernel launches issued since the last
  * reset, measured with CUDA events on the launching stream; reset != 0
  * clears the counters after reading. */
