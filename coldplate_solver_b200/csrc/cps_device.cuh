@@ -1510,7 +1510,7 @@ __device__ __forceinline__ int ring_place(int q, int& a, int& b) {
 }
 
 // Tiles per CTA the two builds of the form hold: few (small designs) and what
-// two CTAs per SM leave of shared memory.
+// two CTAs per SM leave of shared memory with 8 x 32 tiles.
 constexpr int kFewTiles = 2;
 template <typename T>
 struct PcgTileCount {
@@ -1676,6 +1676,7 @@ __device__ __forceinline__ int pcg_tiles(const DesignView& d, Group& g, double* 
 // which no phase writes, are read and count for nothing: the caller keeps them
 // finite (contexts and cps_solve_noalloc clear them).
 // ---------------------------------------------------------------------------
+// Tiles per CTA, sized like PcgTileCount.
 template <typename T>
 struct PcgStreamCount {
   static constexpr int value = sizeof(T) == 8 ? 30 : 55;
@@ -1809,8 +1810,8 @@ __device__ __forceinline__ int pcg_stream(const DesignView& d, Group& g, double*
 }
 
 // ---------------------------------------------------------------------------
-// The same iterations for a design with one tile per CTA and at most 128 tiles,
-// by the first 16 CTAs alone, which are one thread-block cluster; the other
+// The same iterations for a design with one tile per CTA and at most 128 tiles
+// (112 on B200, where seven clusters are resident at one CTA per SM), by the first 16 CTAs alone, which are one thread-block cluster; the other
 // CTAs wait for the outcome at one grid barrier.  On such designs an iteration
 // is two grid reductions of about 1.9 us with 0.6 us of work between them, and
 // a cluster reduces through distributed shared memory in a quarter of that.
@@ -2708,14 +2709,26 @@ __host__ __device__ constexpr size_t tile_smem_bytes() {
   return t > q ? t : q;
 }
 
-// Dynamic shared memory of a kernel that carries `Carry`, and of the monitored
-// one, whose pressure-drop windows (window_values doubles at most) use the
-// buffers after phase D.
+// The pressure-drop monitor's window + slope_window at most, in values: what
+// callers have been told since the windows were first kept in the kernels'
+// shared memory, per tile shape and precision.  They use the buffers after
+// phase D and need somewhat more than those (101 instead of 95 KB, FP64,
+// 8 x 32 tiles).
 template <typename T>
 __host__ __device__ constexpr size_t window_values() {
-  constexpr size_t R = PcgTileCount<T>::value, kM = sizeof(T) == 4 ? R : 1;
-  return sizeof(T) * (kThreads * (6 * R + 2 * kM) + R * (2 * kHalo + kTileI + kTileJ)) / sizeof(double);
+  constexpr bool mixed = sizeof(T) == 4;
+  return kTileJ == 16 ? (mixed ? 13248 : 12384) : kTileJ == 32 ? (mixed ? 13488 : 12664) : (mixed ? 14328 : 13644);
 }
+// Two CTAs per SM (228 KB, 1 KB per CTA reserved, up to 4 KB declared
+// statically), except in mixed precision with 4 x 64 tiles, where pcg_stream's
+// p alone takes 117 KB: one.
+template <typename T>
+constexpr bool kTwoCtasFit = 2 * ((window_values<T>() * sizeof(double) > tile_smem_bytes<T>()
+                                       ? window_values<T>() * sizeof(double)
+                                       : tile_smem_bytes<T>()) + 5 * 1024) <= 228 * 1024;
+static_assert(CPS_MIN_BLOCKS != 2 || (kTwoCtasFit<double> && (kTwoCtasFit<float> || kTileJ == 64)), "two CTAs per SM");
+
+// Dynamic shared memory of a kernel that carries `Carry`, and of the monitored one.
 template <typename T, int Carry, bool Monitor>
 __host__ __device__ constexpr size_t kernel_smem_bytes() {
   // one CTA per SM for the cluster form: its 16 CTAs on 16 SMs, and the other
