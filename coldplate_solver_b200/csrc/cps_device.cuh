@@ -296,11 +296,12 @@ __device__ __forceinline__ double select(bool c, double a, double b) {
 }
 // One Newton step of y towards 1/b.
 __device__ __forceinline__ double recip_step(double b, double y) { return __fma_rn(y, __fma_rn(-b, y, 1.0), y); }
-// The last step, with the exception.
+// The last step, with the exception: for all ones y is the power of two and
+// y + y e the middle between it and its neighbour; y's last bit set in the
+// product tips it over and is lost in the rounding elsewhere.
 __device__ __forceinline__ double recip_last(double b, double y) {
-  y = recip_step(b, y);
-  const bool ones = ((__double2hiint(b) | ~0xfffff) & __double2loint(b)) == -1;
-  return __hiloint2double(__double2hiint(y), ones ? 1 : __double2loint(y));
+  const double up = __hiloint2double(__double2hiint(y), __double2loint(y) | 1);
+  return __fma_rn(up, __fma_rn(-b, y, 1.0), y);
 }
 // 1/b from y within a few units of its last place.
 __device__ __forceinline__ double recip_from(double b, double y) { return recip_last(b, recip_step(b, y)); }
