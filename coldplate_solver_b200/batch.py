@@ -46,8 +46,12 @@ def mode_candidates(device: int = 0) -> List[dict]:
 
 def default_mode(device: int = 0) -> dict:
     """Placement used when none is given: groups of as many CTAs as the device
-    has SMs (two designs in flight at two CTAs per SM), which measured fastest
-    on the 16- and 64-design mixes; the autotuner picks per workload."""
+    has SMs (two designs in flight at two CTAs per SM), which was fastest on
+    mixes while the PCG ran from global memory.  With its state on chip half
+    as many CTAs per group are faster (B200, ms of 12 early / 100 late outer
+    iterations, groups of 148 -> 74: 8 designs up to 512 wide 55.5 / 16.1 ->
+    31.1 / 11.3, 16 up to 1024 wide 138 / 46 -> 107 / 38, 6 up to 700 wide
+    41.7 / 10.9 -> 29.0 / 9.3); the autotuner picks per workload."""
     try:
         import torch
         return {"group_ctas": torch.cuda.get_device_properties(device).multi_processor_count}
