@@ -25,17 +25,21 @@ __global__ void __launch_bounds__(cps::kThreads, Carry == cps::kCluster ? 1 : CP
   const bool clustered = Carry == cps::kCluster && blockIdx.x < cps::kClusterCtas;  // the cluster that runs the PCG
   if (clustered) cps::cluster_enter();
   cps::SweepHint hint{2, 2};
-  int r = 0;
-  for (int it = 0; it < rc.n_outer && r == 0; ++it) {
-    r = cps::outer_iteration<T, cps::GridGroup, Monitor, Pseudo, Carry>(
+  for (int it = 0; it < rc.n_outer; ++it) {
+    const int r = cps::outer_iteration<T, cps::GridGroup, Monitor, Pseudo, Carry>(
         d, g, smem, tile_smem, out, it + 1 == rc.n_outer, rc.stop_on_conv != 0, rc.eps, rc.iter0 + it,
         rc.dplog ? rc.dplog + (size_t)4 * it : nullptr, rc.dp_converged, &s_pr, &hint);
-    if (r >= 0 && blockIdx.x == 0 && threadIdx.x == 0) {
+    if (r < 0) {
+      if (clustered && r != cps::kLeft) cps::cluster_leave(true);
+      return;
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
       for (int k = 0; k < 8; ++k) rc.hist[(size_t)it * 8 + k] = out[k];
       *rc.n_done = it + 1;
     }
+    if (r == 1) break;
   }
-  if (clustered && r != cps::kLeft) cps::cluster_leave(r < 0);
+  if (clustered) cps::cluster_leave(false);
 }
 
 // Batched solves: each cluster takes the next design from the queue and runs
