@@ -2148,7 +2148,7 @@ __device__ int pcg_single_reduction(const DesignView& d, Group& g, double* smem,
   if (d.maxPIter <= 0) return 0;
   auto inv_diag = [&](size_t q, double r) -> double {
     const double dg = (double)w.pdiag[q];
-    return (fabs(dg) > 1e-20) ? div_rn(r, dg) : r;
+    return select(fabs(dg) > 1e-20, div_rn(r, dg), r);
   };
   // w0 = A u0 and delta0 = (w0, u0) come from phase C
   double gam = gamma0;
