@@ -753,6 +753,37 @@ struct GridGroup {
   }
 };
 
+__device__ __forceinline__ void cluster_arrive() {
+  __syncwarp();  // .aligned: by all lanes together
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
+// The CTAs of a cluster read and write one another's shared memory, so none of
+// them leaves the kernel while another may still do so.  A CTA whose wait
+// failed (anywhere in the outer iteration) tells the others through a word in
+// their shared memory and arrives at the cluster barrier; they meet it at the
+// next one they pass, wherever that is, look at the word there and leave too.
+// Every CTA calls enter (or sets the word before a barrier) before any of them
+// may fail.
+constexpr int kLeft = -2;  // outer_iteration: the PCG's cluster has left together
+constexpr unsigned kStay = 0xffffffffu;
+__shared__ unsigned s_cluster_leave;  // kStay, or the barrier at which to leave
+__device__ __forceinline__ bool cluster_leaving(unsigned barrier = kStay - 1) {
+  return *(volatile unsigned*)&s_cluster_leave <= barrier;
+}
+__device__ __forceinline__ void cluster_enter() {
+  if (threadIdx.x == 0) s_cluster_leave = kStay;
+  cluster_arrive();
+  cluster_wait();
+}
+__device__ __forceinline__ void cluster_leave(bool failed, unsigned barrier = 0) {
+  cg::cluster_group cl = cg::this_cluster();
+  if (failed && threadIdx.x < cl.num_blocks()) *cl.map_shared_rank(&s_cluster_leave, threadIdx.x) = barrier;
+  cluster_arrive();
+  cluster_wait();
+}
+
 // ---------------------------------------------------------------------------
 // Group of CTAs working on one design: one thread-block cluster.  The cluster
 // barrier is a hardware barrier with release/acquire semantics at cluster
@@ -763,10 +794,15 @@ struct ClusterGroup {
   int* status;        // the current design's status word
   unsigned rank, nblk;
   unsigned redCount;
+  unsigned barriers;  // passed in this launch (same in every CTA)
+  bool left;          // the last one was where the cluster leaves
 
+  // Returns false when the CTA must return, as all of the cluster do.
   __device__ bool sync() {
     cg::this_cluster().sync();
-    return true;
+    ++barriers;
+    left = cluster_leaving(barriers);
+    return !left;
   }
 
   template <int K, unsigned MaxMask>
@@ -778,8 +814,8 @@ struct ClusterGroup {
 #pragma unroll
       for (int k = 0; k < K; ++k) slot[k] = v[k];
     }
+    if (!sync()) return false;
     cg::cluster_group cl = cg::this_cluster();
-    cl.sync();
     double acc[K];
 #pragma unroll
     for (int k = 0; k < K; ++k) acc[k] = 0.0;
@@ -1887,32 +1923,6 @@ __device__ __forceinline__ void fold_tiles(const double* p0, const double* p1, i
   s0 = a;
   s1 = b;
 }
-__device__ __forceinline__ void cluster_arrive() {
-  __syncwarp();  // .aligned: by all lanes together
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-
-// The cluster's CTAs store into one another's shared memory, so none of them
-// leaves the kernel while another may still do so.  A CTA whose wait failed
-// (anywhere in the outer iteration) tells the others here and arrives at the
-// cluster barrier; they meet it there, at the end of their own run or in
-// pcg_cluster, whose first barrier ends the PCG when the word is set
-// (kLeft).  Every CTA of the cluster calls enter before any of them stores
-// to another and leave unless it got kLeft.
-constexpr int kLeft = -2;  // outer_iteration: the cluster has left together
-__shared__ int s_cluster_leave;
-__device__ __forceinline__ void cluster_enter() {
-  if (threadIdx.x == 0) s_cluster_leave = 0;
-  cluster_arrive();
-  cluster_wait();
-}
-__device__ __forceinline__ void cluster_leave(bool failed) {
-  if (failed && threadIdx.x < kClusterCtas) *cg::this_cluster().map_shared_rank(&s_cluster_leave, threadIdx.x) = 1;
-  cluster_arrive();
-  cluster_wait();
-}
-
 template <typename T>
 __device__ __forceinline__ int pcg_cluster(const DesignView& d, int rank, char* tbuf, double alpha0, double rz,
                                            double beta) {
@@ -2017,10 +2027,16 @@ __device__ __forceinline__ int pcg_cluster(const DesignView& d, int rank, char* 
     }
     cluster_arrive();
     cluster_wait();
-    if (it == 1 && *(volatile int*)&s_cluster_leave) return kLeft;
+    if (it == 1 && cluster_leaving()) return kLeft;
     double pAp, unused;
     fold_tiles(S.part1, S.part1, tiles, pAp, unused);
-    if (fabs(pAp) < 1e-20) break;
+    if (fabs(pAp) < 1e-20) {
+      if (it == 1) {  // nobody is past this before all have read the word above
+        cluster_arrive();
+        cluster_wait();
+      }
+      break;
+    }
     const double alpha = div_uniform(rz, pAp);
     if (works) {
       double vr[R], vz[R];

@@ -56,12 +56,13 @@ __global__ void __launch_bounds__(cps::kThreads) cps_cluster_kernel(const cps::B
   __shared__ double out[8];
   extern __shared__ __align__(128) char tile_smem[];
   cps::cg::cluster_group cl = cps::cg::this_cluster();
-  cps::ClusterGroup g{redbuf, nullptr, cl.block_rank(), cl.num_blocks(), 0u};
+  cps::ClusterGroup g{redbuf, nullptr, cl.block_rank(), cl.num_blocks(), 0u, 0u, false};
   if (!cps::tile_buffer_fits(tile_smem, cps::tile_smem_bytes<T>(), &results[0].status)) return;
+  if (threadIdx.x == 0) cps::s_cluster_leave = cps::kStay;
   cps::tma_barriers_init();
   for (;;) {
     if (g.rank == 0 && threadIdx.x == 0) s_next = atomicAdd(queue, 1);
-    cl.sync();
+    g.sync();
     const int idx = *cl.map_shared_rank(&s_next, 0);
     if (idx >= n_items) break;
     const int id = order[idx];
@@ -83,6 +84,10 @@ __global__ void __launch_bounds__(cps::kThreads) cps_cluster_kernel(const cps::B
       const int r = cps::outer_iteration<T, cps::ClusterGroup, false, Options, Carry>(
           item.view, g, smem, tile_smem, out, it + 1 == item.n_outer, item.stop_on_conv != 0, item.eps, item.iter0 + it,
           nullptr, nullptr, &s_pr, &hint);
+      if (r < 0) {  // a bounded wait expired here or in another CTA; the design's status says so
+        if (!g.left) cps::cluster_leave(true, g.barriers + 1);
+        return;
+      }
       done = it + 1;
       if (g.rank == 0 && threadIdx.x == 0 && item.hist && it < item.hist_cap)
         for (int k = 0; k < 8; ++k) item.hist[(size_t)it * 8 + k] = out[k];
@@ -94,7 +99,7 @@ __global__ void __launch_bounds__(cps::kThreads) cps_cluster_kernel(const cps::B
       res->converged = (done > 0 && conv <= item.eps) ? 1 : 0;
       for (int k = 0; k < 8; ++k) res->last[k] = out[k];
     }
-    cl.sync();  // s_item, s_next and the reduction ring are reused next round
+    if (!g.sync()) return;  // s_item, s_next and the reduction ring are reused next round
   }
   cl.sync();    // no CTA leaves while another may still read its shared memory
 }
