@@ -292,25 +292,57 @@ struct PlaneOut {
   int rows, cols;
 };
 
-// Copy planes to the caller's memory through the pinned stage, in chunks of
-// rows: while one chunk's rows are written out the next chunks are on their
-// way, and for more than kThreadedDownload bytes several threads write (the
-// caller's memory is usually freshly allocated, and its page faults take
-// longer than the copies).  All eight fields, one thread and one plane at a
-// time -> now: 8 MB of a 500 x 250 design 2.7 -> 1.5 ms, 32 MB of 1000 x 500
-// 9.1 -> 3.1 ms, 134 MB of 2048 x 1024 30.3 -> 7.4 ms.  Slots below
-// kDownloadSlot spend their time in the calls.
-constexpr size_t kThreadedDownload = size_t(4) << 20, kDownloadSlot = size_t(64) << 10;
+// Rows [row, row + rows) of a plane, from the stage to the caller's memory.
+void write_out(const PlaneOut& pl, int row, int rows, const double* src, int layout) {
+  if (layout == CPS_COL_MAJOR) {
+    for (int i = 0; i < rows; ++i)
+      for (int j = 0; j < pl.cols; ++j) pl.dst[(size_t)j * pl.rows + row + i] = src[(size_t)i * pl.cols + j];
+  } else {
+    std::memcpy(pl.dst + (size_t)row * pl.cols, src, sizeof(double) * (size_t)rows * pl.cols);
+  }
+}
+
+// Copy planes to the caller's memory through the pinned stage.  Planes below
+// kPipelinedPlane go one at a time; larger ones in chunks of rows: while one
+// chunk's rows are written out the next chunks are on their way.  Several
+// threads write where that takes longer than their start: the caller's memory
+// is often freshly allocated, and its page faults take longer than the copies;
+// columns are written element by element.  B200's host, us for all eight
+// fields, one plane at a time -> this rule: 40 x 24 98 -> 98 (150 in chunks),
+// 200 x 100 173 -> 173 (199), 340 x 170 382 -> 345; 700 x 350 into fresh
+// memory 2512 -> 1688, into used memory 1249 -> 1073 (8 threads 1560 and 1270);
+// 1000 x 500 fresh 6317 -> 2854, used 2507 -> 1940, by columns 6457 -> 2435.
+// Slots below kDownloadSlot spend their time in the calls.
+constexpr size_t kPipelinedPlane = size_t(384) << 10, kDownloadSlot = size_t(64) << 10;
 constexpr int kDownloadThreads = 8, kDownloadDepth = 2;
+
+int download_threads(size_t bytes, int layout) {
+  const size_t mb = bytes >> 20;
+  return layout == CPS_COL_MAJOR ? (mb >= 4 ? kDownloadThreads : 1)
+                                 : (mb >= 24 ? kDownloadThreads : mb >= 12 ? kDownloadThreads / 2 : 1);
+}
 
 bool download_planes(cps_ctx* c, const PlaneOut* planes, int n, int layout) {
   size_t bytes = 0;
   for (int k = 0; k < n; ++k) bytes += planes[k].dst ? sizeof(double) * (size_t)planes[k].rows * planes[k].cols : 0;
   if (bytes == 0) return true;
   const size_t stage = (size_t)(c->M + 1) * (c->N + 1);
-  int threads = 1;
-  if (bytes > kThreadedDownload)
-    threads = std::max(1, std::min({kDownloadThreads, (int)std::thread::hardware_concurrency() / 2,
+  if (stage * sizeof(double) < kPipelinedPlane) {
+    for (int k = 0; k < n; ++k) {
+      const PlaneOut& pl = planes[k];
+      const size_t w = sizeof(double) * pl.cols;
+      if (!pl.dst) continue;
+      if (!cuda_ok(c, cudaMemcpy2DAsync(c->hstage, w, pl.src, (size_t)c->P * 8, w, pl.rows, cudaMemcpyDeviceToHost, c->stream),
+                   "download") ||
+          !cuda_ok(c, cudaStreamSynchronize(c->stream), "download sync"))
+        return false;
+      write_out(pl, 0, pl.rows, c->hstage, layout);
+    }
+    return true;
+  }
+  int threads = download_threads(bytes, layout);
+  if (threads > 1)
+    threads = std::max(1, std::min({threads, (int)std::thread::hardware_concurrency() / 2,
                                     (int)(stage * sizeof(double) / (kDownloadDepth * kDownloadSlot))}));
   // slots of at least one row each (M >= 3: four rows at least)
   int depth = threads > 1 ? kDownloadDepth : 4;
@@ -348,13 +380,7 @@ bool download_planes(cps_ctx* c, const PlaneOut* planes, int n, int layout) {
       if ((e = cudaEventSynchronize(ev[q])) != cudaSuccess) break;
       const Chunk& h = chunks[m];
       const PlaneOut& pl = planes[h.plane];
-      const double* src = at(q);
-      if (layout == CPS_COL_MAJOR) {
-        for (int i = 0; i < h.rows; ++i)
-          for (int j = 0; j < pl.cols; ++j) pl.dst[(size_t)j * pl.rows + h.row + i] = src[(size_t)i * pl.cols + j];
-      } else {
-        std::memcpy(pl.dst + (size_t)h.row * pl.cols, src, sizeof(double) * (size_t)h.rows * pl.cols);
-      }
+      write_out(pl, h.row, h.rows, at(q), layout);
       if (next < chunks.size()) {
         issue(next, q);
         next += threads;
