@@ -305,21 +305,22 @@ void write_out(const PlaneOut& pl, int row, int rows, const double* src, int lay
 // Copy planes to the caller's memory through the pinned stage.  Planes below
 // kPipelinedPlane go one at a time; larger ones in chunks of rows: while one
 // chunk's rows are written out the next chunks are on their way.  Several
-// threads write where that takes longer than their start: the caller's memory
-// is often freshly allocated, and its page faults take longer than the copies;
-// columns are written element by element.  B200's host, us for all eight
-// fields, one plane at a time -> this rule: 40 x 24 98 -> 98 (150 in chunks),
-// 200 x 100 173 -> 173 (199), 340 x 170 382 -> 345; 700 x 350 into fresh
-// memory 2512 -> 1688, into used memory 1249 -> 1073 (8 threads 1560 and 1270);
-// 1000 x 500 fresh 6317 -> 2854, used 2507 -> 1940, by columns 6457 -> 2435.
-// Slots below kDownloadSlot spend their time in the calls.
+// threads write from 4 MB on: memory that the caller has just allocated (every
+// call through the Python binding) takes longer to fault in than to copy, and
+// columns are written element by element.  By rows into memory already in use
+// each thread costs more than it saves below about 14 MB, hence the ramp.
+// B200's host, us for all eight fields by rows, used / fresh memory, one plane
+// at a time -> this rule (-> chunks always, eight threads from 4 MB): 40 x 24
+// 85 / 92 -> 85 / 92 (116 / 122), 500 x 250 700 / 1485 -> 780 / 705 (920 / 920),
+// 700 x 350 1260 / 2800 -> 1100 / 1110 (1185 / 1250), 1000 x 500 2490 / 7400 ->
+// 1730 / 2070 (1710 / 1980).  Slots below kDownloadSlot spend
+// their time in the calls.
 constexpr size_t kPipelinedPlane = size_t(384) << 10, kDownloadSlot = size_t(64) << 10;
 constexpr int kDownloadThreads = 8, kDownloadDepth = 2;
 
 int download_threads(size_t bytes, int layout) {
-  const size_t mb = bytes >> 20;
-  return layout == CPS_COL_MAJOR ? (mb >= 4 ? kDownloadThreads : 1)
-                                 : (mb >= 24 ? kDownloadThreads : mb >= 12 ? kDownloadThreads / 2 : 1);
+  if (bytes < size_t(4) << 20) return 1;
+  return layout == CPS_COL_MAJOR ? kDownloadThreads : (int)std::min<size_t>(kDownloadThreads, 2 + bytes / (size_t(5) << 19));
 }
 
 bool download_planes(cps_ctx* c, const PlaneOut* planes, int n, int layout) {
