@@ -313,8 +313,8 @@ void write_out(const PlaneOut& pl, int row, int rows, const double* src, int lay
 // at a time -> this rule (-> chunks always, eight threads from 4 MB): 40 x 24
 // 85 / 92 -> 85 / 92 (116 / 122), 500 x 250 700 / 1485 -> 780 / 705 (920 / 920),
 // 700 x 350 1260 / 2800 -> 1100 / 1110 (1185 / 1250), 1000 x 500 2490 / 7400 ->
-// 1730 / 2070 (1710 / 1980).  Slots below kDownloadSlot spend
-// their time in the calls.
+// 1730 / 2070 (1710 / 1980).  Slots below kDownloadSlot spend their time in
+// the calls.
 constexpr size_t kPipelinedPlane = size_t(384) << 10, kDownloadSlot = size_t(64) << 10;
 constexpr int kDownloadThreads = 8, kDownloadDepth = 2;
 
